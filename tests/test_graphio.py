@@ -250,3 +250,57 @@ def test_files_written_on_the_device_pass_the_reference_checker(tmp_path):
     assert c.returncode == 0 and c.stdout.strip() == "", c.stdout
     h.close()
     g.close()
+
+
+def _symmetric(n, lists):
+    """The library's rule in Python: ascending lists, every edge with its reverse."""
+    have = [set(x) for x in lists]
+    return all(x == sorted(x) for x in lists) and all(u in have[v] for u, x in enumerate(lists) for v in x)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,fault", [(1, None), (2, None), (40, None), (1500, None), (1500, "heavy"), (1500, "light"),
+                                     (1500, "equal"), (1500, "unsorted"), (1500, "duplicates"), (1500, "loops"),
+                                     (1500, "swapped")])
+def test_symmetry_detection(cuda_device, n, fault):
+    """A hub over several warps' segments, isolated vertices, and each way to miss a reverse edge: the one that a
+    lookup finds (from the heavier end), the ones that only the counts show, both at once."""
+    import pbbsbench_b200 as pb
+
+    rng = np.random.default_rng(n)
+    have = [set() for _ in range(n)]
+    for u, v in [(0, v) for v in range(1, n, 2)] + [tuple(rng.integers(0, max(1, n - 3), 2)) for _ in range(2 * n)]:
+        if u != v:
+            have[int(u)].add(int(v))
+            have[int(v)].add(int(u))
+    lists = [sorted(x) for x in have]
+    by_deg = sorted(range(1, n), key=lambda v: (len(lists[v]), v))
+    if fault == "heavy":  # the light end's entry is gone: the hub's edge finds no reverse
+        lists[lists[0][5]].remove(0)
+    elif fault == "light":  # the hub's entry is gone: the light end's edge is left over
+        lists[0].pop(5)
+    elif fault == "equal":
+        u, v = next((u, v) for u in range(1, n) for v in lists[u] if len(lists[u]) == len(lists[v]) and u < v)
+        lists[v].remove(u)
+    elif fault == "unsorted":
+        v = by_deg[-1]
+        lists[v][0], lists[v][-1] = lists[v][-1], lists[v][0]
+    elif fault == "duplicates":
+        for v in (0, by_deg[-1], by_deg[len(by_deg) // 2]):
+            lists[v] = sorted(lists[v] + lists[v][:3])
+    elif fault == "loops":
+        for v in (0, by_deg[-1], n - 1):
+            lists[v] = sorted(lists[v] + [v])
+    elif fault == "swapped":  # one entry too many and one too few: the counts agree, a lookup does not
+        lists[0].pop(5)
+        w = next(v for v in range(1, n) if lists[v] and 0 not in lists[v])
+        lists[0] = sorted(lists[0] + [w])
+    off = np.concatenate([[0], np.cumsum([len(x) for x in lists])]).astype(np.uint32)
+    edg = np.array([v for x in lists for v in x] + [0], np.uint32)
+    h, fl = ctypes.c_void_p(), ctypes.c_uint32()
+    L = pb.lib()
+    pb.check(L.pbg_graph_upload(off.ctypes.data, edg.ctypes.data, n, int(off[-1]), 2, ctypes.byref(h)))
+    pb.check(L.pbg_graph_flags(h, ctypes.byref(fl)))
+    pb.check(L.pbg_graph_free(h))
+    assert bool(fl.value & 1) == _symmetric(n, lists)
+    assert _symmetric(n, lists) == (fault in (None, "duplicates", "loops"))
