@@ -134,3 +134,57 @@ def test_long_lists_checked_through_their_tails(cuda_device):
     assert _oracle_verdict(off, edg, 0, cases["parent at the right level, not a neighbour"], True) == h
     assert _oracle_verdict(off, edg, 0, cases["parent at the right level, not a neighbour"], False) == NONE
     dg.close()
+
+
+def _levels_verdict(off, edg, srcs, rows):
+    """First failing (row, vertex) of the level predicate with its level and lowest neighbour level, in numpy."""
+    n = len(off) - 1
+    deg = np.diff(off).astype(np.int64)
+    for r in range(len(srcs)):
+        lv = rows[r].astype(np.int64)
+        lv[lv == 255] = n
+        mn = np.full(n, n, np.int64)
+        np.minimum.at(mn, np.repeat(np.arange(n), deg), lv[edg])
+        ok = ((lv == n) & (mn == n)) | ((mn < n) & (lv == mn + 1))
+        ok[srcs[r]] = lv[srcs[r]] == 0
+        if not ok.all():
+            v = int(np.argmin(ok))
+            return {"bad_vertex": v, "row": r, "level": int(lv[v]), "min_neighbor_level": int(mn[v])}
+    return None
+
+
+@pytest.mark.parametrize("n", [200, 257, 4099])
+@pytest.mark.parametrize("k", [1, 4, 5, 17, 33, 64, 67])
+def test_levels_rows_in_strips(cuda_device, n, k):
+    """Row counts on both sides of every strip width, an odd n, lists of over 64 and over 320 entries (one and several
+    tail pieces), unreached vertices, and faults whose only evidence is in a list's tail."""
+    rng = np.random.default_rng(n * 100 + k)
+    us, vs = [], []
+    for hub, d in ((0, min(n - 9, 900)), (1, min(n - 9, 90))):
+        to = rng.choice(np.arange(2, n - 6), d - 2, replace=False)
+        us += [hub] * len(to)
+        vs += to.tolist()
+    a, b = rng.integers(2, n - 6, 3 * n), rng.integers(2, n - 6, 3 * n)
+    off, edg = O.csr_symmetric(n, np.array(us + a.tolist(), np.uint32), np.array(vs + b.tolist(), np.uint32))
+    dg = pb.DeviceGraph.upload(off, edg)
+    srcs = rng.choice(np.nonzero(np.diff(off))[0], k).astype(np.uint32)
+    srcs[0] = 0
+    rows = np.stack([np.minimum(O.bfs_levels(off, edg, int(s)).astype(np.int64), 255).astype(np.uint8) for s in srcs])
+
+    def both(x):
+        got = dg.levels_check(srcs, torch.from_numpy(x.reshape(-1)).cuda())
+        want = _levels_verdict(off, edg, srcs, x)
+        if want is None:
+            assert got["bad_vertex"] == NONE
+        else:
+            assert got == want
+        return want
+
+    assert both(rows) is None
+    for r in sorted({0, k // 2, k - 1}):
+        for v, to in ((int(srcs[r]), 1), (int(edg[off[1] - 1]), 3), (n - 1, 7), (int(edg[off[1] - 1]), 255),
+                      (int(edg[off[2] - 1]), 0), (int(rng.integers(0, n)), 254), (2, n if n < 255 else 254)):
+            bad = rows.copy()
+            bad[r, v] = to if bad[r, v] != to else to ^ 1
+            assert both(bad) is not None or n < 255
+    dg.close()
