@@ -30,9 +30,10 @@
 // Parent rules:
 //   ANY: claim by atomicOr on bm[cur] in place; the winner writes parent.
 //   MIN/MAX: every frontier edge into a vertex not in bm[cur] (read-only this
-//     level) does atomicMin/atomicMax on parent; the claim that decides who
-//     enqueues v goes to bm[cur^1], which holds level <= L-1 and receives the
-//     frontier's own bits from the threads expanding it; then cur flips.
+//     level) does atomicMin/atomicMax on parent; the one that finds it unset
+//     enqueues v and sets its bit in bm[cur^1], which holds level <= L-1 and
+//     receives the frontier's own bits from the threads expanding it; then
+//     cur flips.
 //   Bottom-up scans N(v) ascending (MAX: descending) and stops at the first
 //   frontier neighbour, which is the min (max) because lists are sorted.
 //
@@ -43,6 +44,7 @@
 // Graphs whose largest degree is below the chunk degree run bfs_lean, the
 // same search without the chunk queue (see its comment).
 #include <cuda_runtime.h>
+#include <stddef.h>
 #include <stdint.h>
 
 #include <algorithm>
@@ -60,6 +62,8 @@ using dev::globaltimer;
 using dev::ld_relaxed_u64;
 constexpr uint32_t CHUNK = 256;  // edges per chunk task: 8 per lane of a warp
 constexpr int PER_LANE = 8;      // independent loads each lane keeps in flight
+constexpr uint32_t CONV = 3;     // BfsCtrl::conv as a slot index
+static_assert(offsetof(BfsCtrl, conv) == offsetof(BfsCtrl, slot) + CONV * sizeof(LevelSlot), "conv follows the slots");
 constexpr unsigned long long BIG_SHIFT = 40;
 constexpr unsigned long long BIG_MASK = (1ull << BIG_SHIFT) - 1;
 
@@ -126,6 +130,32 @@ __device__ __forceinline__ void load_ranges(const BfsArgs& a, const uint32_t (&v
   }
 }
 
+// Which of the paired arrays a level reads and writes, as bits of one word:
+// the pointers are selected from the launch arguments where they are used,
+// which costs a select each and keeps some 20 registers free for the loops.
+// The 1024-thread kernels are held to 64 registers: with this and 32-bit
+// per-thread sums they spill 136-156 bytes (bfs_lean 48-72) instead of
+// 184-204 (60-88); torus 160^3 1.677 -> 1.622 ms, rMat 2^24 0.562 -> 0.547 ms,
+// rMat 2^12 53.2 -> 51.2 us.
+struct Level {
+  uint32_t bits;  // 0: output queues are q0/qr0/qb0 (else q1/qr1/qb1); 1: bm1 is the visited bitmap
+  uint32_t slot;  // counters of the frontier produced (3: conv)
+  uint32_t next;  // level number of what is found
+  __device__ __forceinline__ LevelSlot* out(const BfsArgs& a) const { return a.ctrl->slot + slot; }
+  __device__ __forceinline__ uint32_t* q(const BfsArgs& a) const { return (bits & 1u) ? a.q0 : a.q1; }
+  __device__ __forceinline__ uint2* qr(const BfsArgs& a) const { return (bits & 1u) ? a.qr0 : a.qr1; }
+  __device__ __forceinline__ uint4* qb(const BfsArgs& a) const { return (bits & 1u) ? a.qb0 : a.qb1; }
+  __device__ __forceinline__ const uint32_t* qin(const BfsArgs& a) const { return (bits & 1u) ? a.q1 : a.q0; }
+  __device__ __forceinline__ const uint2* qrin(const BfsArgs& a) const { return (bits & 1u) ? a.qr1 : a.qr0; }
+  __device__ __forceinline__ const uint4* qbin(const BfsArgs& a) const { return (bits & 1u) ? a.qb1 : a.qb0; }
+  __device__ __forceinline__ const uint32_t* vis(const BfsArgs& a) const { return (bits & 2u) ? a.bm1 : a.bm0; }
+  // ANY claims in the visited bitmap itself, MIN/MAX in the other one
+  template <int MODE>
+  __device__ __forceinline__ uint32_t* claim(const BfsArgs& a) const {
+    return ((bits & 2u) != 0) == (MODE == MODE_ANY) ? a.bm1 : a.bm0;
+  }
+};
+
 // Warp-collective append of up to K vertices per lane (cand[i] for the set
 // bits i of `win`) to the next frontier.  Vertices with degree >= chunk_deg
 // go to the chunk queue as (v, begin, end, first chunk) with their number of
@@ -135,9 +165,8 @@ __device__ __forceinline__ void load_ranges(const BfsArgs& a, const uint32_t (&v
 // contiguous, and chunk numbering follows slot order across warps because
 // slot and chunk counters move in one 64-bit atomic.
 template <int K>
-__device__ __forceinline__ void emit_k(const BfsArgs& a, LevelSlot* out, uint32_t* qout, uint2* qrout,
-                                       uint4* qbout, const uint32_t (&cand)[K], unsigned win,
-                                       unsigned long long& degacc, const uint32_t (&ob)[K],
+__device__ __forceinline__ void emit_k(const BfsArgs& a, const Level& lv, const uint32_t (&cand)[K], unsigned win,
+                                       uint32_t& degacc, const uint32_t (&ob)[K],
                                        const uint32_t (&oe)[K]) {
   if (!__any_sync(FULL, win != 0)) return;
   const int lane = threadIdx.x & 31;
@@ -162,12 +191,12 @@ __device__ __forceinline__ void emit_k(const BfsArgs& a, LevelSlot* out, uint32_
   const uint32_t ts = __shfl_sync(FULL, ps, 31), tc = __shfl_sync(FULL, pc, 31), tch = __shfl_sync(FULL, pch, 31);
   unsigned long long bs = 0, bc = 0;
   if (lane == 0) {
-    if (ts) bs = atomicAdd(&out->nmain, (unsigned long long)ts);
-    if (tc) bc = atomicAdd(&out->big, ((unsigned long long)tc << BIG_SHIFT) | tch);
+    if (ts) bs = atomicAdd(&lv.out(a)->nmain, (unsigned long long)ts);
+    if (tc) bc = atomicAdd(&lv.out(a)->big, ((unsigned long long)tc << BIG_SHIFT) | tch);
   }
   bs = __shfl_sync(FULL, bs, 0);
   bc = __shfl_sync(FULL, bc, 0);
-  unsigned long long ps_pos = bs + ps - ns;
+  uint32_t ps_pos = (uint32_t)bs + ps - ns;
   uint32_t pc_pos = (uint32_t)(bc >> BIG_SHIFT) + pc - nc;
   uint32_t chunk = (uint32_t)(bc & BIG_MASK) + pch - nch;
   // pass 2: write
@@ -177,14 +206,14 @@ __device__ __forceinline__ void emit_k(const BfsArgs& a, LevelSlot* out, uint32_
       const uint32_t b = ob[i], e = oe[i];
       if ((chunked >> i) & 1u) {
         if (pc_pos < a.big_cap)
-          qbout[pc_pos] = make_uint4(cand[i], b, e, chunk);
+          lv.qb(a)[pc_pos] = make_uint4(cand[i], b, e, chunk);
         else
           atomicOr(&a.ctrl->sync.error, ERR_QUEUE);
         pc_pos++;
         chunk += (e - b + CHUNK - 1) / CHUNK;
       } else {
-        qout[ps_pos] = cand[i];
-        qrout[ps_pos] = make_uint2(b, e);
+        lv.q(a)[ps_pos] = cand[i];
+        lv.qr(a)[ps_pos] = make_uint2(b, e);
         ps_pos++;
         // the next level reads this list: start it on its way from HBM to L2
         if (e > b) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.edges + b));
@@ -194,62 +223,75 @@ __device__ __forceinline__ void emit_k(const BfsArgs& a, LevelSlot* out, uint32_
 }
 
 // Top-down claims of up to K neighbours v[i] (set bits of `act`) by the
-// lane's vertex u.  Every load and atomic of the K candidates is issued before
+// lane's vertex u, and the adjacency ranges (ob, oe) of the candidates that
+// may be won.  Every load and atomic of the K candidates is issued before
 // any store that depends on one, so the K round trips overlap instead of
 // running one after another.  Returns the bits of the candidates this lane
 // enqueues.
+// MIN/MAX test the read-only snapshot of the level's visited set first and
+// load ranges for the unvisited only; the reduction that finds the parent
+// unset is the claim.  Large levels are bound by the L1's rate of about one
+// request a clock and SM, and most of their edges lead to visited vertices:
+// a directed graph of 2 M vertices (22.8 M edges reached, MAX) took 0.592 ms
+// with ranges for every edge and a second atomic for every unvisited one,
+// 0.557 ms with these and the arguments selected late (Level).
 template <int MODE, int K>
-__device__ __forceinline__ unsigned td_claim_k(const BfsArgs& a, const uint32_t* vis, uint32_t* claim, uint32_t u,
-                                               const uint32_t (&v)[K], unsigned act, uint32_t next_level) {
-  unsigned live = act;
-  if (MODE != MODE_ANY) {
-    // MIN/MAX test the read-only snapshot of the level's visited set first
-    uint32_t w[K];
+__device__ __forceinline__ unsigned td_claim_k(const BfsArgs& a, const Level& lv, uint32_t u,
+                                               const uint32_t (&v)[K], unsigned act, uint32_t (&ob)[K],
+                                               uint32_t (&oe)[K]) {
+  uint32_t old[K];
+  unsigned win = 0;
+  if (MODE == MODE_ANY) {
+    load_ranges(a, v, act, ob, oe);
 #pragma unroll
-    for (int i = 0; i < K; i++) w[i] = ((act >> i) & 1u) ? vis[v[i] >> 5] : 0u;
+    for (int i = 0; i < K; i++) old[i] = ((act >> i) & 1u) ? atomicOr(lv.claim<MODE>(a) + (v[i] >> 5), 1u << (v[i] & 31)) : FULL;
 #pragma unroll
     for (int i = 0; i < K; i++)
-      if ((w[i] >> (v[i] & 31)) & 1u) live &= ~(1u << i);
-#pragma unroll
-    for (int i = 0; i < K; i++) {
-      if ((live >> i) & 1u) {
-        if (MODE == MODE_MIN)
-          atomicMin(a.parent + v[i], u);
-        else
-          atomicMax(reinterpret_cast<int*>(a.parent) + v[i], (int)u);
-      }
-    }
-  }
-  uint32_t old[K];
-#pragma unroll
-  for (int i = 0; i < K; i++) old[i] = ((live >> i) & 1u) ? atomicOr(claim + (v[i] >> 5), 1u << (v[i] & 31)) : FULL;
-  unsigned win = 0;
-#pragma unroll
-  for (int i = 0; i < K; i++)
-    if (!((old[i] >> (v[i] & 31)) & 1u)) win |= 1u << i;
-  if (MODE == MODE_ANY) {
+      if (!((old[i] >> (v[i] & 31)) & 1u)) win |= 1u << i;
 #pragma unroll
     for (int i = 0; i < K; i++)
       if ((win >> i) & 1u) a.parent[v[i]] = u;
+  } else {
+    unsigned live = act;
+    uint32_t w[K];
+#pragma unroll
+    for (int i = 0; i < K; i++) w[i] = ((act >> i) & 1u) ? lv.vis(a)[v[i] >> 5] : 0u;
+#pragma unroll
+    for (int i = 0; i < K; i++)
+      if ((w[i] >> (v[i] & 31)) & 1u) live &= ~(1u << i);
+    load_ranges(a, v, live, ob, oe);
+#pragma unroll
+    for (int i = 0; i < K; i++) {
+      old[i] = 0;
+      if ((live >> i) & 1u)
+        old[i] = (MODE == MODE_MIN) ? atomicMin(a.parent + v[i], u)
+                                    : (uint32_t)atomicMax(reinterpret_cast<int*>(a.parent) + v[i], (int)u);
+    }
+#pragma unroll
+    for (int i = 0; i < K; i++) {
+      if (old[i] == PBG_NONE) {
+        win |= 1u << i;
+        atomicOr(lv.claim<MODE>(a) + (v[i] >> 5), 1u << (v[i] & 31));
+      }
+    }
   }
   if (a.level && win) {
 #pragma unroll
     for (int i = 0; i < K; i++)
-      if ((win >> i) & 1u) a.level[v[i]] = next_level;
+      if ((win >> i) & 1u) a.level[v[i]] = lv.next;
   }
   return win;
 }
 
 // One CHUNK-edge piece of a long list, expanded by a whole warp.
 template <int MODE>
-__device__ __forceinline__ void td_chunk(const BfsArgs& a, const uint4& ent, uint32_t c_local, const uint32_t* vis,
-                                         uint32_t* claim, LevelSlot* out, uint32_t* qout, uint2* qrout,
-                                         uint4* qbout, uint32_t next_level, unsigned long long& degacc) {
+__device__ __forceinline__ void td_chunk(const BfsArgs& a, const uint4& ent, uint32_t c_local, const Level& lv,
+                                         uint32_t& degacc) {
   const int lane = threadIdx.x & 31;
   const uint32_t u = ent.x;
   const uint32_t cb = ent.y + c_local * CHUNK;
   const uint32_t ce = min(ent.z, cb + CHUNK);
-  if (MODE != MODE_ANY && c_local == 0 && lane == 0) atomicOr(claim + (u >> 5), 1u << (u & 31));
+  if (MODE != MODE_ANY && c_local == 0 && lane == 0) atomicOr(lv.claim<MODE>(a) + (u >> 5), 1u << (u & 31));
   uint32_t v[PER_LANE];
   unsigned act = 0;
 #pragma unroll
@@ -262,26 +304,23 @@ __device__ __forceinline__ void td_chunk(const BfsArgs& a, const uint4& ent, uin
     }
   }
   uint32_t ob[PER_LANE], oe[PER_LANE];
-  load_ranges(a, v, act, ob, oe);
-  const unsigned win = td_claim_k<MODE, PER_LANE>(a, vis, claim, u, v, act, next_level);
-  emit_k<PER_LANE>(a, out, qout, qrout, qbout, v, win, degacc, ob, oe);
+  const unsigned win = td_claim_k<MODE, PER_LANE>(a, lv, u, v, act, ob, oe);
+  emit_k<PER_LANE>(a, lv, v, win, degacc, ob, oe);
 }
 
 // 32 short lists (degree < chunk_deg), one per lane, PER_LANE edges a step.
 template <int MODE>
-__device__ __forceinline__ void td_small(const BfsArgs& a, uint32_t tile, const uint32_t* qin,
-                                         const uint2* qrin, unsigned long long nmain, const uint32_t* vis,
-                                         uint32_t* claim, LevelSlot* out, uint32_t* qout, uint2* qrout,
-                                         uint4* qbout, uint32_t next_level, unsigned long long& degacc) {
+__device__ __forceinline__ void td_small(const BfsArgs& a, uint32_t tile, uint32_t nmain, const Level& lv,
+                                         uint32_t& degacc) {
   const int lane = threadIdx.x & 31;
-  const unsigned long long idx = (unsigned long long)tile * 32 + lane;
+  const uint32_t idx = tile * 32 + lane;  // n < 2^31
   uint32_t u = 0, b = 0, e = 0;
   if (idx < nmain) {
-    u = qin[idx];
-    const uint2 r = qrin[idx];  // range stored by the claimer: no offsets load
+    u = lv.qin(a)[idx];
+    const uint2 r = lv.qrin(a)[idx];  // range stored by the claimer: no offsets load
     b = r.x;
     e = r.y;
-    if (MODE != MODE_ANY) atomicOr(claim + (u >> 5), 1u << (u & 31));
+    if (MODE != MODE_ANY) atomicOr(lv.claim<MODE>(a) + (u >> 5), 1u << (u & 31));
   }
   const uint32_t maxd = __reduce_max_sync(FULL, e - b);
   for (uint32_t k0 = 0; k0 < maxd; k0 += PER_LANE) {
@@ -297,40 +336,36 @@ __device__ __forceinline__ void td_small(const BfsArgs& a, uint32_t tile, const 
       }
     }
     uint32_t ob[PER_LANE], oe[PER_LANE];
-    load_ranges(a, v, act, ob, oe);
-    const unsigned win = td_claim_k<MODE, PER_LANE>(a, vis, claim, u, v, act, next_level);
-    emit_k<PER_LANE>(a, out, qout, qrout, qbout, v, win, degacc, ob, oe);
+    const unsigned win = td_claim_k<MODE, PER_LANE>(a, lv, u, v, act, ob, oe);
+    emit_k<PER_LANE>(a, lv, v, win, degacc, ob, oe);
   }
 }
 
 // Top-down level: chunk tasks first (edge-balanced over every warp of the
 // grid), then 32-entry tiles of short lists.
 template <int MODE>
-__device__ void td_level(const BfsArgs& a, const uint32_t* qin, const uint2* qrin, unsigned long long nmain,
-                         const uint4* qbin, uint32_t nbig, uint32_t nchunks, const uint32_t* vis, uint32_t* claim,
-                         LevelSlot* out, uint32_t* qout, uint2* qrout, uint4* qbout, uint32_t next_level,
-                         unsigned long long& degacc) {
+__device__ void td_level(const BfsArgs& a, uint32_t nmain, uint32_t nbig, uint32_t nchunks, const Level& lv,
+                         uint32_t& degacc) {
   // tasks go round-robin over blocks first, so a small level still uses
   // every SM's load/store pipeline
   const uint32_t gw = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
   const uint32_t tw = (gridDim.x * blockDim.x) >> 5;
-  const unsigned long long tasks = nchunks + (nmain + 31) / 32;
+  const unsigned long long tasks = (unsigned long long)nchunks + (nmain + 31) / 32;
   for (unsigned long long t = gw; t < tasks; t += tw) {
     if (t < nchunks) {
       const uint32_t c = (uint32_t)t;
       uint32_t lo = 0, hi = nbig - 1;
       while (lo < hi) {
         const uint32_t mid = (lo + hi + 1) >> 1;
-        if (qbin[mid].w <= c)
+        if (lv.qbin(a)[mid].w <= c)
           lo = mid;
         else
           hi = mid - 1;
       }
-      const uint4 ent = qbin[lo];
-      td_chunk<MODE>(a, ent, c - ent.w, vis, claim, out, qout, qrout, qbout, next_level, degacc);
+      const uint4 ent = lv.qbin(a)[lo];
+      td_chunk<MODE>(a, ent, c - ent.w, lv, degacc);
     } else {
-      td_small<MODE>(a, (uint32_t)(t - nchunks), qin, qrin, nmain, vis, claim, out, qout, qrout, qbout, next_level,
-                     degacc);
+      td_small<MODE>(a, (uint32_t)(t - nchunks), nmain, lv, degacc);
     }
   }
 }
@@ -350,8 +385,8 @@ __device__ void td_level(const BfsArgs& a, const uint32_t* qin, const uint2* qri
 // registers.
 template <int MODE>
 __device__ __forceinline__ void bu_word(const BfsArgs& a, const uint32_t* vin, uint32_t* vout, uint32_t next_level,
-                                        uint32_t w, uint32_t word, uint32_t b, uint32_t e, unsigned long long& cnt,
-                                        unsigned long long& degacc) {
+                                        uint32_t w, uint32_t word, uint32_t b, uint32_t e, uint32_t& cnt,
+                                        uint32_t& degacc) {
   constexpr int PROBES = 4;
   constexpr uint32_t LSHARE = 16;
   const int lane = threadIdx.x & 31;
@@ -437,7 +472,7 @@ __device__ __forceinline__ void bu_word(const BfsArgs& a, const uint32_t* vin, u
 
 template <int MODE>
 __device__ void bu_level(const BfsArgs& a, const uint32_t* vin, uint32_t* vout, uint32_t next_level,
-                         unsigned long long& cnt, unsigned long long& degacc) {
+                         uint32_t& cnt, uint32_t& degacc) {
   const int lane = threadIdx.x & 31;
   const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t tw = (gridDim.x * blockDim.x) >> 5;
@@ -471,12 +506,11 @@ __device__ void bu_level(const BfsArgs& a, const uint32_t* vin, uint32_t* vout, 
 // Rebuilds the frontier queues from the bitmap difference after a bottom-up
 // level (the sparse form of the dense frontier, as pack_index does in
 // ligraLight.h:132).  Lane l of a warp handles word w0 + l.
-__device__ void dense_to_queue(const BfsArgs& a, const uint32_t* before, const uint32_t* after, LevelSlot* out,
-                               uint32_t* qout, uint2* qrout, uint4* qbout) {
+__device__ void dense_to_queue(const BfsArgs& a, const uint32_t* before, const uint32_t* after, const Level& lv) {
   const int lane = threadIdx.x & 31;
   const uint32_t gw = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
   const uint32_t tw = (gridDim.x * blockDim.x) >> 5;
-  unsigned long long dummy = 0;
+  uint32_t dummy = 0;
   for (uint32_t w0 = gw * 32; w0 < a.nwords; w0 += tw * 32) {
     const uint32_t w = w0 + lane;
     uint32_t diff = (w < a.nwords) ? (after[w] & ~before[w]) : 0u;
@@ -494,7 +528,7 @@ __device__ void dense_to_queue(const BfsArgs& a, const uint32_t* before, const u
       }
       uint32_t ob[PER_LANE], oe[PER_LANE];
       load_ranges(a, v, act, ob, oe);
-      emit_k<PER_LANE>(a, out, qout, qrout, qbout, v, act, dummy, ob, oe);
+      emit_k<PER_LANE>(a, lv, v, act, dummy, ob, oe);
     }
   }
 }
@@ -597,16 +631,10 @@ __global__ void __launch_bounds__(BLOCK, BLOCK == 256 ? 4 : 1) bfs_persistent(Bf
       }
     }
 
-    uint32_t* qin = (L & 1) ? a.q1 : a.q0;
-    uint2* qrin = (L & 1) ? a.qr1 : a.qr0;
-    uint2* qrout = (L & 1) ? a.qr0 : a.qr1;
-    uint32_t* qout = (L & 1) ? a.q0 : a.q1;
-    uint4* qbin = (L & 1) ? a.qb1 : a.qb0;
-    uint4* qbout = (L & 1) ? a.qb0 : a.qb1;
     uint32_t* bcur = cur ? a.bm1 : a.bm0;
     uint32_t* both = cur ? a.bm0 : a.bm1;
     if (bu) {
-      unsigned long long cnt = 0, degacc = 0;
+      uint32_t cnt = 0, degacc = 0;
       bu_level<MODE>(a, bcur, both, L + 1, cnt, degacc);
       const unsigned long long bc = block_sum(cnt);
       const unsigned long long bd = block_sum(degacc);
@@ -618,7 +646,7 @@ __global__ void __launch_bounds__(BLOCK, BLOCK == 256 ? 4 : 1) bfs_persistent(Bf
     } else {
       if (prev_bu) {
         // the frontier came from a bottom-up level: build its queues first
-        dense_to_queue(a, both, bcur, &c->conv, qin, qrin, qbin);
+        dense_to_queue(a, both, bcur, Level{(L & 1u) ^ 1u, CONV, L});
         ok = dev::grid_barrier(&c->sync, ERR_BARRIER_TIMEOUT, bar_epoch);
         if (!ok) break;
         if (threadIdx.x == 0) {
@@ -635,10 +663,9 @@ __global__ void __launch_bounds__(BLOCK, BLOCK == 256 ? 4 : 1) bfs_persistent(Bf
         if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(&c->sync.error, ERR_QUEUE);
         break;
       }
-      uint32_t* claim = (MODE == MODE_ANY) ? bcur : both;
-      unsigned long long degacc = 0;
-      td_level<MODE>(a, qin, qrin, nmain, qbin, nbig, (uint32_t)(big & BIG_MASK), bcur, claim, out, qout, qrout,
-                     qbout, L + 1, degacc);
+      uint32_t degacc = 0;
+      td_level<MODE>(a, (uint32_t)nmain, nbig, (uint32_t)(big & BIG_MASK),
+                     Level{(L & 1u) | (cur << 1), (L + 1) % 3, L + 1}, degacc);
       const unsigned long long bd = block_sum(degacc);
       if (threadIdx.x == 0 && bd) atomicAdd(&out->deg, bd);
       if (MODE != MODE_ANY) cur ^= 1u;
@@ -672,9 +699,9 @@ __global__ void __launch_bounds__(BLOCK, BLOCK == 256 ? 4 : 1) bfs_persistent(Bf
 
 // Appends the winners (bits of `win`) of a step to the next queue, one atomic
 // per warp.
-__device__ __forceinline__ void lean_emit(const BfsArgs& a, LevelSlot* out, uint32_t* qout, uint2* qrout,
+__device__ __forceinline__ void lean_emit(const BfsArgs& a, const Level& lv,
                                           const uint32_t (&cand)[PER_LANE], unsigned win,
-                                          unsigned long long& degacc, const uint32_t (&ob)[PER_LANE],
+                                          uint32_t& degacc, const uint32_t (&ob)[PER_LANE],
                                           const uint32_t (&oe)[PER_LANE]) {
   if (!__any_sync(FULL, win != 0)) return;
   const int lane = threadIdx.x & 31;
@@ -682,15 +709,15 @@ __device__ __forceinline__ void lean_emit(const BfsArgs& a, LevelSlot* out, uint
   const uint32_t ps = warp_incl_scan(ns);
   const uint32_t ts = __shfl_sync(FULL, ps, 31);
   unsigned long long b0 = 0;
-  if (lane == 0) b0 = atomicAdd(&out->nmain, (unsigned long long)ts);
+  if (lane == 0) b0 = atomicAdd(&lv.out(a)->nmain, (unsigned long long)ts);
   unsigned long long pos = __shfl_sync(FULL, b0, 0) + ps - ns;
 #pragma unroll
   for (int i = 0; i < PER_LANE; i++) {
     if ((win >> i) & 1u) {
       const uint32_t b = ob[i], e = oe[i];
       degacc += e - b;
-      qout[pos] = cand[i];
-      qrout[pos] = make_uint2(b, e);
+      lv.q(a)[pos] = cand[i];
+      lv.qr(a)[pos] = make_uint2(b, e);
       pos++;
       // the next level reads this list: start it on its way from HBM to L2
       if (e > b) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.edges + b));
@@ -700,19 +727,17 @@ __device__ __forceinline__ void lean_emit(const BfsArgs& a, LevelSlot* out, uint
 
 // 32 queue entries, one per lane, PER_LANE edges a step.
 template <int MODE>
-__device__ __forceinline__ void lean_tile(const BfsArgs& a, uint32_t tile, const uint32_t* qin, const uint2* qrin,
-                                          unsigned long long nq, const uint32_t* vis, uint32_t* claim,
-                                          LevelSlot* out, uint32_t* qout, uint2* qrout, uint32_t next_level,
-                                          unsigned long long& degacc) {
+__device__ __forceinline__ void lean_tile(const BfsArgs& a, uint32_t tile, uint32_t nq, const Level& lv,
+                                          uint32_t& degacc) {
   const int lane = threadIdx.x & 31;
-  const unsigned long long idx = (unsigned long long)tile * 32 + lane;
+  const uint32_t idx = tile * 32 + lane;  // n < 2^31
   uint32_t u = 0, b = 0, e = 0;
   if (idx < nq) {
-    u = qin[idx];
-    const uint2 r = qrin[idx];  // range stored by the claimer: no offsets load
+    u = lv.qin(a)[idx];
+    const uint2 r = lv.qrin(a)[idx];  // range stored by the claimer: no offsets load
     b = r.x;
     e = r.y;
-    if (MODE != MODE_ANY) atomicOr(claim + (u >> 5), 1u << (u & 31));
+    if (MODE != MODE_ANY) atomicOr(lv.claim<MODE>(a) + (u >> 5), 1u << (u & 31));
   }
   const uint32_t maxd = __reduce_max_sync(FULL, e - b);
   for (uint32_t k0 = 0; k0 < maxd; k0 += PER_LANE) {
@@ -728,9 +753,8 @@ __device__ __forceinline__ void lean_tile(const BfsArgs& a, uint32_t tile, const
       }
     }
     uint32_t ob[PER_LANE], oe[PER_LANE];
-    load_ranges(a, v, act, ob, oe);
-    const unsigned win = td_claim_k<MODE, PER_LANE>(a, vis, claim, u, v, act, next_level);
-    lean_emit(a, out, qout, qrout, v, win, degacc, ob, oe);
+    const unsigned win = td_claim_k<MODE, PER_LANE>(a, lv, u, v, act, ob, oe);
+    lean_emit(a, lv, v, win, degacc, ob, oe);
   }
 }
 
@@ -815,14 +839,9 @@ __global__ void __launch_bounds__(1024, 1) bfs_lean(BfsArgs a) {
         tdl++;
       }
     }
-    uint32_t* qin = (L & 1) ? a.q1 : a.q0;
-    uint2* qrin = (L & 1) ? a.qr1 : a.qr0;
-    uint2* qrout = (L & 1) ? a.qr0 : a.qr1;
-    uint32_t* qout = (L & 1) ? a.q0 : a.q1;
-    uint4* qbin = (L & 1) ? a.qb1 : a.qb0;
     uint32_t* bcur = cur ? a.bm1 : a.bm0;
     uint32_t* both = cur ? a.bm0 : a.bm1;
-    unsigned long long cnt = 0, degacc = 0;
+    uint32_t cnt = 0, degacc = 0;
     if (bu) {
       bu_level<MODE>(a, bcur, both, L + 1, cnt, degacc);
       cur ^= 1u;
@@ -830,7 +849,7 @@ __global__ void __launch_bounds__(1024, 1) bfs_lean(BfsArgs a) {
       if (prev_bu) {
         // the frontier came from a bottom-up level: build its queue first
         // (every list is short, so nothing goes to the chunk queue)
-        dense_to_queue(a, both, bcur, &c->conv, qin, qrin, qbin);
+        dense_to_queue(a, both, bcur, Level{(L & 1u) ^ 1u, CONV, L});
         ok = dev::grid_barrier(&c->sync, ERR_BARRIER_TIMEOUT, bar_epoch);
         if (!ok) break;
         if (threadIdx.x == 0) s_in[0] = ld_relaxed_u64(&c->conv.nmain);
@@ -842,25 +861,22 @@ __global__ void __launch_bounds__(1024, 1) bfs_lean(BfsArgs a) {
         if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(&c->sync.error, ERR_QUEUE);
         break;
       }
-      uint32_t* claim = (MODE == MODE_ANY) ? bcur : both;
+      const Level lv{(L & 1u) | (cur << 1), (L + 1) % 3, L + 1};
       // tiles go round-robin over blocks first, so a small level still uses
       // every SM's load/store pipeline
       const uint32_t gw = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
       const uint32_t tw = (gridDim.x * blockDim.x) >> 5;
       const unsigned long long tiles = (nq + 31) / 32;
       for (unsigned long long t = gw; t < tiles; t += tw)
-        lean_tile<MODE>(a, (uint32_t)t, qin, qrin, nq, bcur, claim, out, qout, qrout, L + 1, degacc);
+        lean_tile<MODE>(a, (uint32_t)t, (uint32_t)nq, lv, degacc);
       if (MODE != MODE_ANY) cur ^= 1u;
     }
     // per warp: one reduction atomic per counter (no block barrier)
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      cnt += __shfl_down_sync(FULL, cnt, o);
-      degacc += __shfl_down_sync(FULL, degacc, o);
-    }
+    cnt = __reduce_add_sync(FULL, cnt);
+    degacc = __reduce_add_sync(FULL, degacc);
     if ((threadIdx.x & 31) == 0) {
-      if (bu && cnt) atomicAdd(&out->nmain, cnt);  // a count: the frontier is the bitmap difference
-      if (degacc) atomicAdd(&out->deg, degacc);
+      if (bu && cnt) atomicAdd(&out->nmain, (unsigned long long)cnt);  // a count: the frontier is the bitmap difference
+      if (degacc) atomicAdd(&out->deg, (unsigned long long)degacc);
     }
     prev_bu = bu;
     L++;
