@@ -7,9 +7,9 @@
 //
 // Generators restate testData/graphData/{rMatGraph,gridGraph,randLocalGraph}.C
 // with SplitMix64's output mix as the hash (parlay::hash64 is unavailable),
-// and build the symmetric CSR as common/graphUtils.h:54-94 does: drop self
-// loops, add reversed edges, sort by (u, v), drop duplicates, count, scan.
-// The sort is cub::DeviceRadixSort over packed (u << shift | v) keys.
+// and build the symmetric CSR of common/graphUtils.h:54-94: no self loops,
+// both directions, lists ascending, no duplicates.  The sorts are
+// cub::DeviceRadixSort over packed keys (keys_to_graph).
 #include <cub/cub.cuh>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -79,36 +79,35 @@ __global__ void k_validate(const uint32_t* __restrict__ off, const uint32_t* __r
     if (edg[i] >= n) atomicOr(bad, 4u);
 }
 
+// The generators write one key per drawn edge, smaller end first: (min << shift
+// | max).  A self loop becomes `sentinel`, the key of the loop at vertex n - 1,
+// which no edge has and no key exceeds, so it sorts last.
+__device__ __forceinline__ uint64_t edge_key(uint32_t u, uint32_t v, uint32_t shift, uint64_t sentinel) {
+  return u == v ? sentinel : ((uint64_t)min(u, v) << shift) | max(u, v);
+}
+
 // rMat draw for edge i (rMatGraph.C:53-69): start/stride keys from i and the
-// seed hash, one 31-bit draw per level, top level first.
+// seed hash, one 31-bit draw per level, top level first.  The quadrant's two
+// bits come from comparisons without branches: the arms are drawn at random,
+// so a warp took every one of them at every level (2^28 draws of 24 levels:
+// 8.7 ms with branches, 7.5 ms without).
 __global__ void k_gen_rmat(uint64_t m, uint64_t h, uint32_t logn, uint32_t ta, uint32_t tab, uint32_t tabc,
                            uint32_t shift, uint64_t sentinel, uint64_t* __restrict__ keys) {
   const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const uint64_t nth = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t i = tid; i < m; i += nth) {
-    const uint64_t rs = mix64((2 * i) * h);
+    uint64_t x = mix64((2 * i) * h);
     const uint64_t st = mix64((2 * i + 1) * h);
     uint32_t u = 0, v = 0;
+#pragma unroll 4
     for (uint32_t k = 0; k < logn; k++) {
-      const uint32_t half = 1u << (logn - 1 - k);
-      const uint32_t r = (uint32_t)(mix64(rs + (uint64_t)k * st) & 0x7FFFFFFFu);
-      if (r < ta) {
-      } else if (r < tab) {
-        v += half;
-      } else if (r < tabc) {
-        u += half;
-      } else {
-        u += half;
-        v += half;
-      }
+      const uint32_t r = (uint32_t)(mix64(x) & 0x7FFFFFFFu);
+      x += st;
+      const uint32_t low = r >= tab;  // the lower half of the rows
+      u = 2 * u + low;
+      v = 2 * v + ((low ? r >= tabc : r >= ta) ? 1u : 0u);
     }
-    if (u == v) {
-      keys[2 * i] = sentinel;
-      keys[2 * i + 1] = sentinel;
-    } else {
-      keys[2 * i] = ((uint64_t)u << shift) | v;
-      keys[2 * i + 1] = ((uint64_t)v << shift) | u;
-    }
+    keys[i] = edge_key(u, v, shift, sentinel);
   }
 }
 
@@ -126,17 +125,7 @@ __global__ void k_gen_torus(uint32_t dn, const uint32_t* __restrict__ perm, uint
     uint64_t nb[3] = {(((i + 1) % dn) * dn + j) * dn + k, (i * dn + (j + 1) % dn) * dn + k,
                       (i * dn + j) * dn + (k + 1) % dn};
     const uint32_t u = relabel(perm, (uint32_t)l);
-    for (int d = 0; d < 3; d++) {
-      const uint32_t v = relabel(perm, (uint32_t)nb[d]);
-      const uint64_t o = 6 * l + 2 * d;
-      if (u == v) {
-        keys[o] = sentinel;
-        keys[o + 1] = sentinel;
-      } else {
-        keys[o] = ((uint64_t)u << shift) | v;
-        keys[o + 1] = ((uint64_t)v << shift) | u;
-      }
-    }
+    for (int d = 0; d < 3; d++) keys[3 * l + d] = edge_key(u, relabel(perm, (uint32_t)nb[d]), shift, sentinel);
   }
 }
 
@@ -160,8 +149,7 @@ __global__ void k_gen_randlocal(uint32_t n, uint32_t deg, uint32_t w, uint64_t h
       if (j != i) break;
       x = mix64(x);
     }
-    keys[2 * t] = ((uint64_t)i << shift) | j;
-    keys[2 * t + 1] = ((uint64_t)j << shift) | i;
+    keys[t] = edge_key((uint32_t)i, j, shift, sentinel);
   }
 }
 
@@ -258,18 +246,74 @@ __global__ void k_symmetric(const uint32_t* __restrict__ off, const uint32_t* __
   }
 }
 
-// Sorted unique keys -> CSR.  offsets[v] = index of the first key with
-// source >= v; edges[i] = low part of key i.
-__global__ void k_keys_to_csr(const uint64_t* __restrict__ keys, uint64_t m, uint32_t n, uint32_t shift,
+// first[v] = index of the first of the `cnt` sorted keys whose vertex (the
+// key's upper end when HIGH, else its lower bits) is v or above, for v in
+// [0, n].  Key i (i = cnt: the end) fills the vertices after its
+// predecessor's up to its own; the whole warp calls, and fills a long run of
+// vertices without keys together.  Returns key i's vertex.
+template <bool HIGH>
+__device__ __forceinline__ uint32_t fill_first(const uint64_t* __restrict__ keys, uint64_t cnt, uint32_t n,
+                                               uint32_t shift, uint64_t i, uint32_t* __restrict__ first) {
+  constexpr uint32_t FULL = 0xFFFFFFFFu, RUN = 32;
+  const uint64_t vmask = (1ull << shift) - 1;
+  auto vertex = [&](uint64_t k) { return (uint32_t)(HIGH ? k >> shift : k & vmask); };
+  uint32_t v = n, lo = 1, hi = 0;  // nothing to fill past the end
+  if (i <= cnt) {
+    if (i < cnt) v = vertex(keys[i]);
+    lo = i ? vertex(keys[i - 1]) + 1 : 0;
+    hi = v + 1;
+  }
+  const bool longrun = hi > lo && hi - lo > RUN;
+  if (!longrun)
+    for (uint32_t w = lo; w < hi; w++) first[w] = (uint32_t)i;
+  for (unsigned mm = __ballot_sync(FULL, longrun); mm; mm &= mm - 1) {
+    const int l = __ffs(mm) - 1;
+    const uint32_t b = __shfl_sync(FULL, lo, l), e = __shfl_sync(FULL, hi, l), x = __shfl_sync(FULL, (uint32_t)i, l);
+    for (uint32_t w = b + (threadIdx.x & 31); w < e; w += 32) first[w] = x;
+  }
+  return v;
+}
+
+// Keys in (lower end, upper end) order: where each lower end's begin, and a
+// copy of the keys for the second sort.
+__global__ void k_first_lower(const uint64_t* __restrict__ keys, uint64_t cnt, uint32_t n, uint32_t shift,
+                              uint32_t* __restrict__ first, uint64_t* __restrict__ copy) {
+  const uint64_t nth = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t b = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) & ~31ull; b <= cnt; b += nth) {
+    const uint64_t i = b + (threadIdx.x & 31);
+    fill_first<true>(keys, cnt, n, shift, i, first);
+    if (i < cnt) copy[i] = keys[i];
+  }
+}
+
+// Keys in (upper end, lower end) order: where each upper end's begin, and
+// the first part of every list, the neighbours below the vertex.  The list
+// of v starts at below[v] + above[v], so key i's lower end goes to
+// i - below[v] past that, i + above[v].
+__global__ void k_lists_below(const uint64_t* __restrict__ keys, uint64_t cnt, uint32_t n, uint32_t shift,
+                              const uint32_t* __restrict__ above, uint32_t* __restrict__ below,
+                              uint32_t* __restrict__ edg) {
+  const uint64_t nth = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t b = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) & ~31ull; b <= cnt; b += nth) {
+    const uint64_t i = b + (threadIdx.x & 31);
+    const uint32_t v = fill_first<false>(keys, cnt, n, shift, i, below);
+    if (i < cnt) edg[i + above[v]] = (uint32_t)(keys[i] >> shift);
+  }
+}
+
+// The rest of every list, the neighbours above the vertex (keys in (lower,
+// upper) order): past the list's below[v + 1] - below[v] first entries, key
+// i's upper end goes to i + below[v + 1].  Also the offsets.
+__global__ void k_lists_above(const uint64_t* __restrict__ keys, uint64_t cnt, uint32_t n, uint32_t shift,
+                              const uint32_t* __restrict__ above, const uint32_t* __restrict__ below,
                               uint32_t* __restrict__ off, uint32_t* __restrict__ edg) {
   const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const uint64_t nth = (uint64_t)gridDim.x * blockDim.x;
   const uint64_t vmask = (1ull << shift) - 1;
-  for (uint64_t i = tid; i <= m; i += nth) {
-    const uint64_t u = (i < m) ? (keys[i] >> shift) : n;
-    const uint64_t pu = (i == 0) ? 0 : ((keys[i - 1] >> shift) + 1);
-    for (uint64_t w = pu; w <= u && w <= n; w++) off[w] = (uint32_t)i;
-    if (i < m) edg[i] = (uint32_t)(keys[i] & vmask);
+  for (uint64_t v = tid; v <= n; v += nth) off[v] = above[v] + below[v];
+  for (uint64_t i = tid; i < cnt; i += nth) {
+    const uint64_t k = keys[i];
+    edg[i + below[(k >> shift) + 1]] = (uint32_t)(k & vmask);
   }
 }
 
@@ -374,46 +418,93 @@ struct DevBuf {
   }
 };
 
-// Sort 2*m packed keys, drop duplicates and sentinels, build the CSR into g.
-int keys_to_graph(uint64_t* keys, uint64_t nkeys, uint32_t n, uint32_t shift, uint64_t sentinel,
-                  pbg_graph** out, cudaStream_t s, int num_sms) {
-  DevBuf sorted, uniq, nsel, tmp;
-  PBG_CUDA(sorted.alloc(sizeof(uint64_t) * nkeys));
-  PBG_CUDA(uniq.alloc(sizeof(uint64_t) * nkeys));
-  PBG_CUDA(nsel.alloc(sizeof(unsigned long long)));
-  const int end_bit = (int)std::min<uint32_t>(64, 2 * shift + 1);
-  size_t t1 = 0, t2 = 0;
-  PBG_CUDA(cub::DeviceRadixSort::SortKeys(nullptr, t1, keys, sorted.as<uint64_t>(), nkeys, 0, end_bit, s));
-  PBG_CUDA(cub::DeviceSelect::Unique(nullptr, t2, sorted.as<uint64_t>(), uniq.as<uint64_t>(),
-                                     nsel.as<unsigned long long>(), nkeys, s));
-  PBG_CUDA(tmp.alloc(std::max(t1, t2)));
-  size_t tb = std::max(t1, t2);
-  PBG_CUDA(cub::DeviceRadixSort::SortKeys(tmp.p, tb, keys, sorted.as<uint64_t>(), nkeys, 0, end_bit, s));
-  tb = std::max(t1, t2);
-  PBG_CUDA(cub::DeviceSelect::Unique(tmp.p, tb, sorted.as<uint64_t>(), uniq.as<uint64_t>(),
-                                     nsel.as<unsigned long long>(), nkeys, s));
-  unsigned long long nu = 0;
-  PBG_CUDA(cudaMemcpyAsync(&nu, nsel.p, sizeof(nu), cudaMemcpyDeviceToHost, s));
+// The symmetric CSR of the drawn edges: each edge once (keys, smaller end
+// first), sorted by (lower, upper) end with duplicates dropped, then stably
+// by the upper end alone, which gives every vertex's neighbours below it;
+// those above it are the first order's.  Half the keys of a sort of both
+// directions, and the second sort has the upper end's bits only; all scratch
+// is one allocation of two key arrays (keys is the first; the list array, as
+// long as one, is the second sort's third), not four of both directions, since
+// mapping and unmapping memory costs milliseconds a GB.  rMat 2^24 with 2^28
+// draws: 76 ms before, 47 ms now (24 ms of it the sorts' nine passes); 2^12 with 2^16
+// draws, where the allocations count: 2.3 ms before, 1.4 ms now.
+struct KeyScratch {
+  DevBuf buf;
+  uint64_t* keys = nullptr;  // the generator's output: nkeys entries
+  uint64_t* other = nullptr;
+  uint32_t* above = nullptr;  // n + 1 entries each
+  uint32_t* below = nullptr;
+  unsigned long long* count = nullptr;
+  void* tmp = nullptr;
+  size_t tmp_bytes = 0;
+};
+
+int key_scratch(uint64_t nkeys, uint32_t n, uint32_t shift, KeyScratch* ks) {
+  size_t t1 = 0, t2 = 0, t3 = 0;
+  cub::DoubleBuffer<uint64_t> db;
+  uint64_t *in = nullptr, *out = nullptr;
+  unsigned long long* cnt = nullptr;
+  PBG_CUDA(cub::DeviceRadixSort::SortKeys(nullptr, t1, db, nkeys, 0, (int)(2 * shift)));
+  PBG_CUDA(cub::DeviceSelect::Unique(nullptr, t2, in, out, cnt, nkeys));
+  PBG_CUDA(cub::DeviceRadixSort::SortKeys(nullptr, t3, db, nkeys, 0, (int)shift));
+  ks->tmp_bytes = std::max(t1, std::max(t2, t3));
+  auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
+  const size_t kb = up(sizeof(uint64_t) * nkeys), ob = up(sizeof(uint32_t) * ((size_t)n + 1));
+  if (ks->buf.alloc(2 * kb + 2 * ob + 256 + ks->tmp_bytes) != cudaSuccess) {
+    cudaGetLastError();
+    return fail(PBG_ERR_OOM, "generator: key buffer allocation failed");
+  }
+  char* p = ks->buf.as<char>();
+  ks->keys = reinterpret_cast<uint64_t*>(p);
+  ks->other = reinterpret_cast<uint64_t*>(p + kb);
+  ks->above = reinterpret_cast<uint32_t*>(p + 2 * kb);
+  ks->below = reinterpret_cast<uint32_t*>(p + 2 * kb + ob);
+  ks->count = reinterpret_cast<unsigned long long*>(p + 2 * kb + 2 * ob);
+  ks->tmp = p + 2 * kb + 2 * ob + 256;
+  return PBG_OK;
+}
+
+int keys_to_graph(KeyScratch& ks, uint64_t nkeys, uint32_t n, uint32_t shift, uint64_t sentinel, pbg_graph** out,
+                  cudaStream_t s, int num_sms) {
+  cub::DoubleBuffer<uint64_t> db(ks.keys, ks.other);
+  size_t tb = ks.tmp_bytes;
+  PBG_CUDA(cub::DeviceRadixSort::SortKeys(ks.tmp, tb, db, nkeys, 0, (int)(2 * shift), s));
+  uint64_t* uniq = db.Alternate();  // in (lower, upper) order
+  tb = ks.tmp_bytes;
+  PBG_CUDA(cudaMemsetAsync(ks.count, 0, sizeof(*ks.count), s));
+  PBG_CUDA(cub::DeviceSelect::Unique(ks.tmp, tb, db.Current(), uniq, ks.count, nkeys, s));
+  unsigned long long cnt = 0;
+  PBG_CUDA(cudaMemcpyAsync(&cnt, ks.count, sizeof(cnt), cudaMemcpyDeviceToHost, s));
   PBG_CUDA(cudaStreamSynchronize(s));
-  uint64_t m = nu;
-  if (m > 0) {
+  if (cnt > 0) {
     uint64_t last = 0;
-    PBG_CUDA(cudaMemcpy(&last, uniq.as<uint64_t>() + (m - 1), sizeof(last), cudaMemcpyDeviceToHost));
-    if (last == sentinel) m--;
+    PBG_CUDA(cudaMemcpyAsync(&last, uniq + (cnt - 1), sizeof(last), cudaMemcpyDeviceToHost, s));
+    PBG_CUDA(cudaStreamSynchronize(s));
+    if (last == sentinel) cnt--;
   }
   pbg_graph* g = nullptr;
-  int rc = new_handle(n, m, PBG_GRAPH_SYMMETRIC, &g);
+  int rc = new_handle(n, 2 * cnt, PBG_GRAPH_SYMMETRIC, &g);
   if (rc) return rc;
-  k_keys_to_csr<<<grid_for(m + 1, num_sms), 256, 0, g->stream>>>(uniq.as<uint64_t>(), m, n, shift, g->d_offsets,
-                                                                  g->d_edges);
-  cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
-  if (e == cudaSuccess && m == 0) e = cudaMemset(g->d_offsets, 0, sizeof(uint32_t) * ((uint64_t)n + 1));
-  if (e != cudaSuccess) {
-    pbg_graph_free(g);
-    return cuda_fail(e, "CSR build");
-  }
-  rc = finish_graph(g);
+  auto build = [&]() -> int {
+    uint64_t* upper = db.Current();  // its keys are done with: in (upper, lower) order from here on
+    uint64_t* lists = reinterpret_cast<uint64_t*>(g->d_edges);  // 2 * cnt ids, not written yet
+    const bool odd = ((shift + 7) / 8) & 1;  // passes: the second sort ends in `upper` either way
+    cub::DoubleBuffer<uint64_t> d2(odd ? lists : upper, odd ? upper : lists);
+    k_first_lower<<<grid_for(cnt + 1, num_sms), 256, 0, s>>>(uniq, cnt, n, shift, ks.above, d2.Current());
+    PBG_CUDA(cudaGetLastError());
+    size_t t = ks.tmp_bytes;
+    if (cnt) PBG_CUDA(cub::DeviceRadixSort::SortKeys(ks.tmp, t, d2, cnt, 0, (int)shift, s));
+    if (cnt && d2.Current() != upper)  // a small input's sort may take other passes
+      PBG_CUDA(cudaMemcpyAsync(upper, d2.Current(), sizeof(uint64_t) * cnt, cudaMemcpyDeviceToDevice, s));
+    k_lists_below<<<grid_for(cnt + 1, num_sms), 256, 0, s>>>(upper, cnt, n, shift, ks.above, ks.below, g->d_edges);
+    PBG_CUDA(cudaGetLastError());
+    k_lists_above<<<grid_for(std::max<uint64_t>(cnt, n), num_sms), 256, 0, s>>>(uniq, cnt, n, shift, ks.above,
+                                                                               ks.below, g->d_offsets, g->d_edges);
+    PBG_CUDA(cudaGetLastError());
+    PBG_CUDA(cudaStreamSynchronize(s));
+    return finish_graph(g);
+  };
+  rc = build();
   if (rc) {
     pbg_graph_free(g);
     return rc;
@@ -483,24 +574,23 @@ extern "C" int pbg_graph_generate(const pbg_gen_params* p, pbg_graph** out) {
     if (!(p->a >= 0 && p->b >= 0 && p->c >= 0 && p->a + p->b + p->c <= 1.0))
       return fail(PBG_ERR_ARG, "rmat: a + b + c must be <= 1 (rMatGraph.C:44-47)");
     n = 1ull << p->logn;
-    nkeys = 2 * p->samples;
+    nkeys = p->samples;
   } else if (p->kind == PBG_GEN_TORUS3D) {
     if (p->dn < 1) return fail(PBG_ERR_ARG, "torus: dn must be >= 1");
     n = (uint64_t)p->dn * p->dn * p->dn;
-    nkeys = 6 * n;
+    nkeys = 3 * n;
   } else if (p->kind == PBG_GEN_RANDLOCAL) {
     if (p->n < 2) return fail(PBG_ERR_ARG, "randlocal: n must be >= 2");
     if (p->window < 1) return fail(PBG_ERR_ARG, "randlocal: window must be >= 1");
     n = p->n;
-    nkeys = 2ull * p->n * p->degree;
+    nkeys = (uint64_t)p->n * p->degree;
   } else {
     return fail(PBG_ERR_ARG, "unknown generator kind");
   }
   if (n > PBG_MAX_VERTICES)
     return fail(PBG_ERR_ARG, "n must be below 2^31: vertex ids are int (bench/BFS.h:5)");
   const uint32_t shift = std::max<uint32_t>(1, ceil_log2(n));
-  if (2 * shift + 1 > 64) return fail(PBG_ERR_ARG, "graph too large for packed keys");
-  const uint64_t sentinel = 1ull << (2 * shift);
+  const uint64_t sentinel = ((n - 1) << shift) | (n - 1);
 
   int dev = 0, num_sms = 0;
   PBG_CUDA(cudaGetDevice(&dev));
@@ -512,17 +602,15 @@ extern "C" int pbg_graph_generate(const pbg_gen_params* p, pbg_graph** out) {
     ~StreamGuard() { cudaStreamDestroy(s); }
   } sg{s};
 
-  DevBuf keys, perm;
-  cudaError_t e = keys.alloc(sizeof(uint64_t) * nkeys);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    return fail(PBG_ERR_OOM, "generator: key buffer allocation failed");
-  }
-  const int grid = grid_for(nkeys / 2 + 1, num_sms);
+  DevBuf perm;
+  KeyScratch ks;
+  const int rc = key_scratch(nkeys, (uint32_t)n, shift, &ks);
+  if (rc) return rc;
+  const int grid = grid_for(nkeys + 1, num_sms);
   if (p->kind == PBG_GEN_RMAT) {
     const uint64_t h = mix64(p->seed);
     k_gen_rmat<<<grid, 256, 0, s>>>(p->samples, h, p->logn, prob_threshold(p->a), prob_threshold(p->a + p->b),
-                                    prob_threshold(p->a + p->b + p->c), shift, sentinel, keys.as<uint64_t>());
+                                    prob_threshold(p->a + p->b + p->c), shift, sentinel, ks.keys);
   } else if (p->kind == PBG_GEN_TORUS3D) {
     if (p->permute) {
       DevBuf pk, ps, tmp;
@@ -538,13 +626,13 @@ extern "C" int pbg_graph_generate(const pbg_gen_params* p, pbg_graph** out) {
       PBG_CUDA(cudaGetLastError());
       PBG_CUDA(cudaStreamSynchronize(s));
     }
-    k_gen_torus<<<grid, 256, 0, s>>>(p->dn, perm.as<uint32_t>(), shift, sentinel, keys.as<uint64_t>());
+    k_gen_torus<<<grid, 256, 0, s>>>(p->dn, perm.as<uint32_t>(), shift, sentinel, ks.keys);
   } else {
     k_gen_randlocal<<<grid, 256, 0, s>>>(p->n, p->degree, p->window, mix64(p->seed), shift, sentinel,
-                                         keys.as<uint64_t>());
+                                         ks.keys);
   }
   PBG_CUDA(cudaGetLastError());
-  return keys_to_graph(keys.as<uint64_t>(), nkeys, (uint32_t)n, shift, sentinel, out, s, num_sms);
+  return keys_to_graph(ks, nkeys, (uint32_t)n, shift, sentinel, out, s, num_sms);
 }
 
 extern "C" int pbg_graph_info(const pbg_graph* g, uint32_t* n, uint64_t* m, const uint32_t** d_offsets,
