@@ -42,7 +42,8 @@
 // return, the host reports PBG_ERR_TIMEOUT.
 //
 // Graphs whose largest degree is below the chunk degree run bfs_lean, the
-// same search without the chunk queue (see its comment).
+// same search without the chunk queue, and small graphs bfs_small, one block
+// with its state in shared memory (see their comments).
 #include <cuda_runtime.h>
 #include <stddef.h>
 #include <stdint.h>
@@ -895,6 +896,389 @@ __global__ void __launch_bounds__(1024, 1) bfs_lean(BfsArgs a) {
   }
 }
 
+// ---------------------------------------------------------------- small graphs
+// Graphs of at most SMALL_N vertices whose search one block finishes sooner
+// than the grid (small_graph): the same search with the bitmaps, the parents,
+// the levels and the queue in shared memory.  Such a search is a chain of
+// round trips: a level of the grid-wide kernels costs 4-7 us (claims, queue
+// positions, entries and the barrier all through L2), a top-down level here
+// about 2; only offsets and edges are read from memory.
+constexpr uint32_t SMALL_N = 5120;
+constexpr uint64_t SMALL_M = 1u << 18;
+constexpr uint32_t SMALL_T = 1024;
+constexpr uint32_t SMALL_PAD = 64;  // words past the starts that are read, never a start
+constexpr uint16_t NO_LEVEL = 0xFFFF;
+
+// Where the line lies: one SM walks 2-4 edges a ns, so levels of many edges
+// are the grid's (SMALL_M), and it probes for many unvisited vertices one
+// after another (SMALL_N).  Bottom-up levels reread the lists that no probe
+// ends early: they stay short where the average list is (SHORT), or where
+// hubs, SKEW times the average, are soon met.  Grid / one block, us a search:
+// rMat 2^10, 8n 44.6 / 21.7; 2^12, 16n 53.0 / 29.7; 2^12, 30n 49.2 / 45.6;
+// torus 11^3 90 / 78, 17^3 131 / 132 (MAX 145 / 130); randLocal 5101, 3 edges
+// within 60 420 / 131; directed 5101, 61 k edges 70.3 / 70.0, 121 k 129 / 103.
+// Past the line: rMat 2^14, 16n 53 / 71; torus 25^3 207 / 337; randLocal 2001,
+// 8 edges 171 / 222; 5101, 20 edges 81 / 120; directed 16001, 192 k 111 / 189.
+constexpr uint64_t SHORT = 8, SKEW = 16;
+bool small_graph(const pbg_graph* g) {
+  if (g->n > SMALL_N || g->m > SMALL_M) return false;
+  return !(g->flags & PBG_GRAPH_SYMMETRIC) || g->m <= SHORT * g->n || (uint64_t)g->max_degree * g->n >= SKEW * g->m;
+}
+
+size_t small_bytes(uint32_t n, uint32_t nwords) {
+  // parents, queue; bitmaps; starts, list begins and vertices of a queue chunk; levels
+  return sizeof(uint32_t) * (2 * (size_t)n + 2 * nwords + 3 * SMALL_T + SMALL_PAD) + sizeof(uint16_t) * (size_t)n;
+}
+
+struct SmallState {
+  uint32_t* parent;  // [n]
+  uint32_t* q;       // [n]: every vertex enters one frontier, so all of them follow one another
+  uint32_t* vis;     // [nwords]
+  uint32_t* fresh;   // [nwords] found this level (bottom-up, MIN/MAX)
+  // a chunk of the queue, its entries with edges:
+  uint32_t* start;  // [SMALL_T + SMALL_PAD] first position of an entry, PBG_NONE past the last
+  uint32_t* begin;  // [SMALL_T] its list begin less that
+  uint32_t* ent;    // [SMALL_T] its vertex
+  uint16_t* level;   // [n]
+  uint32_t* tail;
+};
+
+// Appends the lanes' found vertices (bits k of `win`: v[k]) to the queue.
+template <int K>
+__device__ __forceinline__ void small_append(const SmallState& s, const uint32_t (&v)[K], unsigned win) {
+  const uint32_t total = __reduce_add_sync(FULL, __popc(win));
+  if (total == 0) return;
+  const int lane = threadIdx.x & 31;
+  uint32_t at = 0;
+  if (lane == 0) at = atomicAdd(s.tail, total);
+  at = __shfl_sync(FULL, at, 0);
+#pragma unroll
+  for (int k = 0; k < K; k++) {
+    const unsigned b = __ballot_sync(FULL, (win >> k) & 1u);
+    if ((win >> k) & 1u) s.q[at + __popc(b & ((1u << lane) - 1u))] = v[k];
+    at += __popc(b);
+  }
+}
+
+// (1 << SMALL_SHIFT | degree) of a queue entry with edges, 0 of one without:
+// one sum counts both (degrees sum to at most SMALL_M, entries to SMALL_T).
+constexpr uint32_t SMALL_SHIFT = 20, SMALL_DEG = (1u << SMALL_SHIFT) - 1;
+static_assert(SMALL_M <= SMALL_DEG && SMALL_T < (1u << (32 - SMALL_SHIFT)), "packed sums");
+__device__ __forceinline__ uint32_t small_pack(uint32_t d) { return d ? (1u << SMALL_SHIFT) | d : 0u; }
+
+// Exclusive prefix sum of x over the block (two syncs); *total = the sum.
+__device__ __forceinline__ uint32_t small_scan(uint32_t x, uint32_t* s_part, uint32_t* total) {
+  const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const uint32_t incl = warp_incl_scan(x);
+  if (lane == 31) s_part[wid] = incl;
+  __syncthreads();
+  const uint32_t part = s_part[lane];
+  const uint32_t sum = warp_incl_scan(part);
+  *total = __shfl_sync(FULL, sum, 31);
+  const uint32_t before = __shfl_sync(FULL, sum - part, wid);
+  __syncthreads();
+  return before + incl - x;
+}
+
+// Expands the queue chunk in s.start / begin / ent: `total` positions, a run
+// of consecutive ones per warp, 32 * K a step.  The entry of a run's first
+// position is searched; from there each window counts the entries that start
+// in it (at most 32: none is empty).
+template <int MODE>
+__device__ __forceinline__ void small_expand(const BfsArgs& a, const SmallState& s, uint32_t total, uint32_t next) {
+  constexpr int K = 4;
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t run = (total + SMALL_T - 1) / SMALL_T * 32;
+  const uint32_t p0 = (threadIdx.x >> 5) * run, p1 = min(total, p0 + run);
+  if (p0 >= total) return;  // warp-uniform
+  uint32_t own = 0;
+#pragma unroll
+  for (uint32_t step = SMALL_T / 2; step; step >>= 1)
+    if (s.start[own + step] <= p0) own += step;
+  for (uint32_t wb = p0; wb < p1; wb += 32 * K) {
+    uint32_t v[K], u[K];
+    unsigned act = 0, win = 0;
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      const uint32_t w = wb + 32 * k;
+      u[k] = v[k] = 0;
+      if (w >= p1) continue;  // warp-uniform
+      const uint32_t rel = s.start[own + 1 + lane] - (w + 1);
+      const unsigned starts = __reduce_or_sync(FULL, rel < 32 ? 1u << rel : 0u);  // bit j: at position w + 1 + j
+      if (w + lane < p1) {
+        const uint32_t my = own + __popc(starts & ((1u << lane) - 1u));
+        u[k] = s.ent[my];
+        v[k] = __ldg(a.edges + (s.begin[my] + w + lane));  // begin - start may have wrapped: add in 32 bits
+        act |= 1u << k;
+      }
+      own += __popc(starts);
+    }
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      const uint32_t bit = 1u << (v[k] & 31);
+      if (!((act >> k) & 1u) || (s.vis[v[k] >> 5] & bit)) continue;
+      bool won;
+      if (MODE == MODE_ANY) {
+        won = !(atomicOr(s.vis + (v[k] >> 5), bit) & bit);
+        if (won) s.parent[v[k]] = u[k];
+      } else {
+        const uint32_t old = MODE == MODE_MIN
+                                 ? atomicMin(s.parent + v[k], u[k])
+                                 : (uint32_t)atomicMax(reinterpret_cast<int*>(s.parent) + v[k], (int)u[k]);
+        won = old == PBG_NONE;
+        if (won) atomicOr(s.fresh + (v[k] >> 5), bit);
+      }
+      if (won) {
+        s.level[v[k]] = (uint16_t)next;
+        win |= 1u << k;
+      }
+    }
+    small_append<K>(s, v, win);
+  }
+}
+
+// Bottom-up level: a warp takes G bitmap words (all of them in one round of
+// the block), a lane one vertex of each, the first LSHARE neighbours by the lane and the rest of longer lists
+// by the warp, as in bu_word.
+template <int MODE>
+__device__ __forceinline__ void small_bottom_up(const BfsArgs& a, const SmallState& s, uint32_t next) {
+  constexpr int G = SMALL_N / SMALL_T, PROBES = 2;
+  constexpr uint32_t LSHARE = 64;
+  const uint32_t lane = threadIdx.x & 31;
+  auto hit = [&](uint32_t x) { return (s.vis[x >> 5] >> (x & 31)) & 1u; };
+  constexpr uint32_t WARPS = SMALL_T / 32;
+  static_assert(G * WARPS * 32 >= SMALL_N, "one round takes every word");
+  const uint32_t w0 = threadIdx.x >> 5, nw = (a.n + 31) / 32;  // words w0, w0 + WARPS, ...
+  if (w0 < nw) {
+    uint32_t b[G], e[G], v[G], p[G];
+    unsigned todo = 0, found = 0;
+#pragma unroll
+    for (int g = 0; g < G; g++) {
+      v[g] = (w0 + WARPS * g) * 32 + lane;
+      b[g] = e[g] = p[g] = 0;
+      if (w0 + WARPS * g < nw && !((s.vis[w0 + WARPS * g] >> lane) & 1u)) {  // the padding past n is marked visited
+        b[g] = __ldg(a.offsets + v[g]);
+        e[g] = __ldg(a.offsets + v[g] + 1);
+        todo |= 1u << g;
+      }
+    }
+    for (uint32_t k0 = 0; k0 < LSHARE; k0 += PROBES) {
+      bool any = false;
+#pragma unroll
+      for (int g = 0; g < G; g++) any |= ((todo & ~found) >> g & 1u) && e[g] - b[g] > k0;
+      if (!__any_sync(FULL, any)) break;
+      uint32_t x[G][PROBES];
+#pragma unroll
+      for (int g = 0; g < G; g++)
+#pragma unroll
+        for (int i = 0; i < PROBES; i++) {
+          x[g][i] = PBG_NONE;
+          if (w0 + WARPS * g < nw && ((todo & ~found) >> g & 1u) && k0 + i < e[g] - b[g])
+            x[g][i] = __ldg(a.edges + (MODE == MODE_MAX ? e[g] - 1 - k0 - i : b[g] + k0 + i));
+        }
+#pragma unroll
+      for (int g = 0; g < G; g++)
+#pragma unroll
+        for (int i = 0; i < PROBES; i++)
+          if (w0 + WARPS * g < nw && x[g][i] != PBG_NONE && !((found >> g) & 1u) && hit(x[g][i])) {
+            found |= 1u << g;
+            p[g] = x[g][i];
+          }
+    }
+#pragma unroll
+    for (int g = 0; g < G; g++) {
+      if (w0 + WARPS * g >= nw) break;  // warp-uniform
+      unsigned mm = __ballot_sync(FULL, ((todo & ~found) >> g & 1u) && e[g] - b[g] > LSHARE);
+      for (; mm; mm &= mm - 1) {
+        const int l = __ffs(mm) - 1;
+        const uint32_t bb = __shfl_sync(FULL, b[g], l), len = __shfl_sync(FULL, e[g], l) - bb;
+        for (uint32_t j = LSHARE; j < len; j += 32) {  // position in scan order (MAX: from the end)
+          const uint32_t q = j + lane;
+          uint32_t x = 0;
+          bool h = false;
+          if (q < len) {
+            x = __ldg(a.edges + (MODE == MODE_MAX ? bb + len - 1 - q : bb + q));
+            h = hit(x);
+          }
+          const unsigned hb = __ballot_sync(FULL, h);
+          if (hb) {
+            const uint32_t f = __shfl_sync(FULL, x, __ffs(hb) - 1);
+            if (lane == l) {
+              found |= 1u << g;
+              p[g] = f;
+            }
+            break;
+          }
+        }
+      }
+      const unsigned nb = __ballot_sync(FULL, (found >> g) & 1u);
+      if (lane == 0 && nb) s.fresh[w0 + WARPS * g] = nb;
+      if ((found >> g) & 1u) {
+        s.parent[v[g]] = p[g];
+        s.level[v[g]] = (uint16_t)next;
+      }
+    }
+    small_append<G>(s, v, found);
+  }
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(SMALL_T, 1) bfs_small(BfsArgs a) {
+  extern __shared__ uint32_t s_mem[];
+  __shared__ uint32_t s_tail, s_part[32];
+  const uint32_t n = a.n, nw = a.nwords, tid = threadIdx.x;
+  SmallState s;
+  s.parent = s_mem;
+  s.q = s.parent + n;
+  s.vis = s.q + n;
+  s.fresh = s.vis + nw;
+  s.start = s.fresh + nw;
+  s.begin = s.start + SMALL_T + SMALL_PAD;
+  s.ent = s.begin + SMALL_T;
+  s.level = reinterpret_cast<uint16_t*>(s.ent + SMALL_T);
+  s.tail = &s_tail;
+  BfsCtrl* c = a.ctrl;
+  if (tid == 0) c->t_start = globaltimer();
+  for (uint32_t v = tid; v < n; v += SMALL_T) {
+    s.parent[v] = PBG_NONE;
+    s.level[v] = NO_LEVEL;
+  }
+  for (uint32_t w = tid; w < nw; w += SMALL_T) {
+    s.vis[w] = a.iso[w] | (w == a.src >> 5 ? 1u << (a.src & 31) : 0u);
+    s.fresh[w] = 0;
+  }
+  if (tid < SMALL_PAD) s.start[SMALL_T + tid] = PBG_NONE;
+  __syncthreads();
+  if (tid == 0) {
+    s.parent[a.src] = a.src;
+    s.level[a.src] = 0;
+    s.q[0] = a.src;
+    s_tail = 1;
+  }
+  __syncthreads();
+  uint32_t head = 0, L = 0, tdl = 0, bul = 0;
+  unsigned long long reached = 0, bumask = 0;
+  bool prev_bu = false;
+  for (;;) {
+    const uint32_t tail = s_tail, nf = tail - head;
+    if (nf == 0) break;
+    // the first SMALL_T entries' lists (all of them, mostly), and the
+    // frontier's out-degree
+    uint32_t u = 0, b = 0, d = 0, rest = 0;
+    if (tid < nf) {
+      u = s.q[head + tid];
+      b = __ldg(a.offsets + u);
+      d = __ldg(a.offsets + u + 1) - b;
+    }
+    for (uint32_t i = SMALL_T + tid; i < nf; i += SMALL_T) {
+      const uint32_t x = s.q[head + i];
+      rest += __ldg(a.offsets + x + 1) - __ldg(a.offsets + x);
+    }
+    uint32_t total = 0, more = 0;
+    uint32_t at = small_scan(small_pack(d), s_part, &total);
+    if (nf > SMALL_T) small_scan(rest, s_part, &more);
+    const uint32_t fdeg = (total & SMALL_DEG) + more;
+    bool bu;
+    if (a.policy == PBG_DIR_TOPDOWN || !a.symmetric)
+      bu = false;
+    else if (a.policy == PBG_DIR_BOTTOMUP)
+      bu = true;
+    else if (!prev_bu)
+      bu = (unsigned long long)nf + fdeg > a.m / a.alpha;
+    else
+      bu = nf > a.n / a.beta;
+    if (tid == 0) {
+      if (L < PBG_TRACE_LEVELS) {
+        c->t_ns[L] = globaltimer();
+        c->t_nf[L] = nf;
+        c->t_deg[L] = fdeg;
+        c->t_bu[L] = bu ? 1u : 0u;
+      }
+      reached += fdeg;
+      if (bu) {
+        bul++;
+        if (L < 64) bumask |= 1ull << L;
+      } else {
+        tdl++;
+      }
+    }
+    if (bu) {
+      small_bottom_up<MODE>(a, s, L + 1);
+    } else {
+      for (uint32_t c0 = 0; c0 < nf; c0 += SMALL_T) {
+        if (c0) {  // a later chunk of a long queue
+          d = 0;
+          if (c0 + tid < nf) {
+            u = s.q[head + c0 + tid];
+            b = __ldg(a.offsets + u);
+            d = __ldg(a.offsets + u + 1) - b;
+          }
+          at = small_scan(small_pack(d), s_part, &total);  // its syncs also end the chunk before
+        }
+        const uint32_t entries = total >> SMALL_SHIFT;
+        if (tid >= entries) s.start[tid] = PBG_NONE;
+        if (d) {
+          const uint32_t r = at >> SMALL_SHIFT, p = at & SMALL_DEG;
+          s.start[r] = p;
+          s.begin[r] = b - p;
+          s.ent[r] = u;
+        }
+        __syncthreads();
+        small_expand<MODE>(a, s, total & SMALL_DEG, L + 1);
+      }
+    }
+    __syncthreads();
+    if (bu || MODE != MODE_ANY) {
+      for (uint32_t w = tid; w < nw; w += SMALL_T) {
+        const uint32_t f = s.fresh[w];
+        if (f) {
+          s.vis[w] |= f;
+          s.fresh[w] = 0;
+        }
+      }
+      __syncthreads();
+    }
+    prev_bu = bu;
+    head = tail;
+    L++;
+  }
+  for (uint32_t v = tid; v < n; v += SMALL_T) {
+    a.parent[v] = s.parent[v];
+    if (a.level) a.level[v] = s.level[v] == NO_LEVEL ? PBG_NONE : (uint32_t)s.level[v];
+  }
+  if (tid == 0) {
+    if (L <= PBG_TRACE_LEVELS) c->t_ns[L] = globaltimer();
+    c->t_end = globaltimer();
+    c->levels = L;
+    c->td_levels = tdl;
+    c->bu_levels = bul;
+    c->final_bm = 0;
+    c->visited = head;
+    c->edges_reached = reached;
+    c->bu_mask = bumask;
+    c->sync.error = 0;
+  }
+}
+
+template <int MODE>
+int launch_small(const BfsArgs& a, cudaStream_t s) {
+  static std::mutex mu;
+  static int dev_of = -1;
+  int dev = 0;
+  PBG_CUDA(cudaGetDevice(&dev));
+  {
+    std::lock_guard<std::mutex> lk(mu);
+    if (dev_of != dev) {
+      PBG_CUDA(cudaFuncSetAttribute(bfs_small<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)small_bytes(SMALL_N, SMALL_N / 32)));
+      dev_of = dev;
+    }
+  }
+  bfs_small<MODE><<<1, SMALL_T, small_bytes(a.n, a.nwords), s>>>(a);
+  PBG_CUDA(cudaGetLastError());
+  return PBG_OK;
+}
+
 template <int MODE>
 int launch_lean(const BfsArgs& a, int num_sms, cudaStream_t s) {
   static std::mutex mu;
@@ -1093,9 +1477,16 @@ int bfs_launch(pbg_graph* g, uint32_t src, const pbg_bfs_opts& o, uint32_t* d_pa
   a.policy = o.direction;
   a.chunk_deg = o.chunk_min_degree;
   a.symmetric = (g->flags & PBG_GRAPH_SYMMETRIC) ? 1u : 0u;
-  PBG_CUDA(cudaMemsetAsync(w.ctrl, 0, sizeof(BfsCtrl), s));
+  const bool small = small_graph(g);
+  if (!small) PBG_CUDA(cudaMemsetAsync(w.ctrl, 0, sizeof(BfsCtrl), s));  // bfs_small writes what is read of it
   PBG_CUDA(cudaEventRecord(w.ev0, s));
-  if (g->max_degree < o.chunk_min_degree) {  // every list short: no chunk queue (bfs_lean)
+  if (small) {
+    switch (o.parent_mode) {
+      case PBG_PARENT_ANY: rc = launch_small<MODE_ANY>(a, s); break;
+      case PBG_PARENT_MIN: rc = launch_small<MODE_MIN>(a, s); break;
+      default: rc = launch_small<MODE_MAX>(a, s); break;
+    }
+  } else if (g->max_degree < o.chunk_min_degree) {  // every list short: no chunk queue (bfs_lean)
     switch (o.parent_mode) {
       case PBG_PARENT_ANY: rc = launch_lean<MODE_ANY>(a, g->num_sms, s); break;
       case PBG_PARENT_MIN: rc = launch_lean<MODE_MIN>(a, g->num_sms, s); break;

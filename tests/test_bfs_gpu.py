@@ -295,3 +295,80 @@ def test_dropin_behind_reference_driver_and_checker(cuda_device, tmp_path):
     assert c.returncode == 0 and c.stdout.strip() == "", c.stdout
     par = O.read_sequence_int(ofile).view(np.uint32)
     assert O.check_bfs(off, edg, 0, par) == -1
+
+
+def _limit_graph(kind, n):
+    """Symmetric graphs (and directed ones) of exactly n vertices, the last few isolated."""
+    rng = np.random.default_rng(n)
+    k = n - 5
+    if kind == "star":  # one list of n - 6 entries, and a second level behind one leaf
+        us, vs = np.zeros(k - 2, np.int64), np.arange(1, k - 1)
+        us, vs = np.append(us, k - 2), np.append(vs, k - 1)
+    elif kind == "path":
+        us, vs = np.arange(k - 1), np.arange(1, k)
+    else:  # skewed: hubs at random ids, many lists of one or two entries
+        p = rng.permutation(k)
+        us, vs = p[(rng.random(6 * k) ** 3 * k).astype(np.int64)], p[(rng.random(6 * k) * k).astype(np.int64)]
+    off, edg = O.csr_symmetric(n, us.astype(np.uint32), vs.astype(np.uint32))
+    if kind == "directed":  # only the edges to a larger id or to a few small ones
+        keep = (np.repeat(np.arange(n), np.diff(off)) < edg) | (edg < 9)
+        off = np.concatenate([[0], np.cumsum(np.add.reduceat(np.append(keep, 0), off[:-1]) * (np.diff(off) > 0))])
+        edg = edg[keep]
+    return off.astype(np.uint32), edg.astype(np.uint32)
+
+
+@pytest.mark.parametrize("n", [7, 33, 1500, 5120, 5121])
+@pytest.mark.parametrize("kind", ["star", "path", "skewed", "directed"])
+def test_one_block_search_and_its_limit(cuda_device, kind, n):
+    """Both sides of the vertex limit of the one-block search, for every parent rule and direction: a frontier of more
+    than a block's threads, a hub, many levels, vertices without out-edges."""
+    off, edg = _limit_graph(kind, n)
+    sym = kind != "directed"
+    dg = pb.DeviceGraph.upload(off, edg, symmetric=sym)
+    deg = np.diff(off)
+    for src in {0, int(np.argmax(deg)), n - 8 if n > 8 else 1, n - 1}:
+        want = O.bfs_levels(off, edg, src)
+        for direction in (pb.DIR_AUTO, pb.DIR_TOPDOWN, pb.DIR_BOTTOMUP)[: 3 if sym else 2]:
+            if kind == "path" and n > 2000 and (src, direction) != (0, pb.DIR_AUTO):
+                continue
+            for mode, rule in ((pb.PARENT_ANY, None), (pb.PARENT_MIN, "min"), (pb.PARENT_MAX, "max")):
+                par, lv, st = dg.bfs(src, parent_mode=mode, direction=direction, levels=True)
+                assert np.array_equal(lv, want), (src, direction, mode)
+                if rule:
+                    assert np.array_equal(par.view(np.uint32), O.bfs_det_parent(off, edg, src, rule)), (src, direction, mode)
+                elif sym:
+                    assert O.check_bfs(off, edg, src, par.view(np.uint32)) == -1, (src, direction)
+                reached = want != pb.NONE
+                assert st["levels"] == int(want[reached].max()) + 1 and st["visited"] == int(reached.sum())
+                assert st["edges_reached"] == int(deg[reached].sum()) and st["error"] == 0
+                assert st["topdown_levels"] + st["bottomup_levels"] == st["levels"]
+                tr = dg.trace()
+                counts = np.bincount(want[reached])
+                assert [t["frontier"] for t in tr] == counts[: len(tr)].tolist()
+                par2, lv2, _ = dg.bfs(src, parent_mode=mode, direction=direction)
+                assert lv2 is None and (rule is None or np.array_equal(par2, par))
+    dg.close()
+
+
+def test_one_block_search_edge_limit(cuda_device):
+    """Complete graphs on both sides of the edge limit (searched as directed: the symmetric ones are the grid's), and
+    even lists on both sides of the average that the one block takes."""
+    for n in (510, 514):  # 259,590 and 263,682 edges around 2^18
+        us, vs = np.triu_indices(n, 1)
+        off, edg = O.csr_symmetric(n, us.astype(np.uint32), vs.astype(np.uint32))
+        for sym in (False, True):
+            dg = pb.DeviceGraph.upload(off, edg, symmetric=sym)
+            for mode, rule in ((pb.PARENT_MIN, "min"), (pb.PARENT_MAX, "max")):
+                par, lv, _ = dg.bfs(5, parent_mode=mode, levels=True)
+                assert np.array_equal(lv, O.bfs_levels(off, edg, 5))
+                assert np.array_equal(par.view(np.uint32), O.bfs_det_parent(off, edg, 5, rule))
+            dg.close()
+    for degree in (3, 4, 5):
+        off, edg = O.randlocal(4000, degree, 90, 2)
+        dg = pb.DeviceGraph.upload(off, edg)
+        for mode, rule in ((pb.PARENT_MIN, "min"), (pb.PARENT_MAX, "max")):
+            for direction in (pb.DIR_AUTO, pb.DIR_BOTTOMUP):
+                par, lv, _ = dg.bfs(5, parent_mode=mode, direction=direction, levels=True)
+                assert np.array_equal(lv, O.bfs_levels(off, edg, 5))
+                assert np.array_equal(par.view(np.uint32), O.bfs_det_parent(off, edg, 5, rule))
+        dg.close()
