@@ -72,10 +72,9 @@ extern "C" int pbg_bfs(pbg_graph* g, uint32_t src, const pbg_bfs_opts* opts, int
   if (level_out && !w.level) PBG_CUDA(cudaMalloc(&w.level, sizeof(uint32_t) * g->n));
   rc = bfs_launch(g, src, o, w.parent, level_out ? w.level : nullptr, g->stream);
   if (rc) return rc;
-  if (parent_out)
-    PBG_CUDA(cudaMemcpyAsync(parent_out, w.parent, sizeof(uint32_t) * g->n, cudaMemcpyDeviceToHost, g->stream));
-  if (level_out)
-    PBG_CUDA(cudaMemcpyAsync(level_out, w.level, sizeof(uint32_t) * g->n, cudaMemcpyDeviceToHost, g->stream));
-  PBG_CUDA(cudaStreamSynchronize(g->stream));
+  const HostCopy out[2] = {{parent_out, w.parent, sizeof(uint32_t) * (size_t)g->n},
+                           {level_out, w.level, sizeof(uint32_t) * (size_t)g->n}};
+  rc = copy_out(out, 2, g->stream);
+  if (rc) return rc;
   return bfs_read_stats(g, stats);
 }

@@ -162,6 +162,15 @@ int bfs_read_stats(pbg_graph* g, pbg_bfs_stats* st);
 int bfs_read_trace(pbg_graph* g, pbg_level_trace* out, uint32_t cap, uint32_t* count);
 void resolve_opts(const pbg_bfs_opts* in, pbg_bfs_opts* out);
 
+// Results to the caller's host memory (copyout.cu): enqueues the copies on
+// `s` (a NULL dst is skipped) and waits until all are on the host.
+struct HostCopy {
+  void* dst;
+  const void* src;
+  size_t bytes;
+};
+int copy_out(const HostCopy* copies, int count, cudaStream_t s);
+
 // Graph handles (graph.cu): a grid of 256-thread blocks for `work` items
 // (at most 16 blocks per SM); a new handle with device arrays for n + 1
 // offsets and m edges; validation of the CSR now on the device (offsets

@@ -486,8 +486,9 @@ extern "C" int pbg_mis(pbg_graph* g, uint8_t* flags_out, pbg_mis_stats* st) {
   int rc = mis_launch(g, g->mis_flags, g->stream);
   if (rc) return rc;
   g->mis_ran = true;
-  PBG_CUDA(cudaMemcpyAsync(flags_out, g->mis_flags, g->n, cudaMemcpyDeviceToHost, g->stream));
-  PBG_CUDA(cudaStreamSynchronize(g->stream));
+  const HostCopy out{flags_out, g->mis_flags, g->n};
+  rc = copy_out(&out, 1, g->stream);
+  if (rc) return rc;
   pbg_mis_stats tmp;
   return mis_read_stats(g, st ? st : &tmp);
 }

@@ -350,8 +350,9 @@ extern "C" int pbg_bfs_multi(pbg_graph* g, const uint32_t* srcs, uint32_t k, con
   pbg_batch_job job{w, srcs, k, w->levels};
   rc = pbg_bfs_batch(g->ms_batch, &job, 1, &o, g->stream);
   if (rc) return rc;
-  PBG_CUDA(cudaMemcpyAsync(levels_out, w->levels, bytes, cudaMemcpyDeviceToHost, g->stream));
-  PBG_CUDA(cudaStreamSynchronize(g->stream));
+  const HostCopy out{levels_out, w->levels, bytes};
+  rc = copy_out(&out, 1, g->stream);
+  if (rc) return rc;
   pbg_batch_stats tmp;
   return pbg_batch_job_stats(g->ms_batch, w, st ? st : &tmp);
 }
