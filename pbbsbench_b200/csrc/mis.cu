@@ -29,7 +29,8 @@
 // those is walked on by the whole warp, 32 a step.  A queue entry carries (vertex, cursor,
 // list end); each warp collects its requeued entries in shared memory and
 // appends them with one atomic per WQ entries.  One grid barrier per round
-// (bounded, device_util.cuh).  When the graph's lists are ascending (checked
+// (bounded, device_util.cuh).  Once the grid has a lane for every undecided
+// vertex, the last round decides them all (wait_out).  When the graph's lists are ascending (checked
 // once per graph), a walk stops at the first neighbour above v.
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -158,7 +159,12 @@ __device__ __forceinline__ uint8_t walk_warp(const MisArgs& a, uint32_t v, uint3
   return IN_SET;
 }
 
-constexpr uint32_t WQ = 64;  // entries of a warp's requeue buffer in shared memory
+// Entries of a warp's requeue buffer in shared memory.  One atomic a flush, on
+// one address, about 1.4 ns each: rMat 2^24 takes 1.49 ms with 32 entries,
+// 1.06 with 64, 1.02 with 96, as much as fits the 64 KB step of shared memory
+// that 64 entries take too (128 entries, in the next step: 1.03, the flags' L1
+// is smaller).
+constexpr uint32_t WQ = 96;
 
 // Appends a warp's buffered entries to the next round's queue (one atomic).
 __device__ __forceinline__ void wq_flush(const uint32_t* wv, const uint2* wc, uint32_t nbuf, LevelSlot* out,
@@ -220,6 +226,71 @@ __device__ __forceinline__ void decide(const MisArgs& a, uint32_t v, uint32_t j,
   __syncwarp();
 }
 
+__device__ __forceinline__ uint8_t ld_flag_fresh(const uint8_t* p) {
+  uint16_t v;
+  asm volatile("ld.relaxed.gpu.global.u8 %0, [%1];" : "=h"(v) : "l"(p) : "memory");
+  return (uint8_t)v;
+}
+
+// The last round: every undecided vertex has a lane of the grid (all blocks
+// are resident), so the lanes keep their vertices and look again at the
+// neighbour each waits for, read from L2, until all are decided, with no
+// queue and no barrier in between.  The smallest undecided vertex decides at
+// its next look, so the wait ends; it is bounded all the same, as a barrier's
+// is.  A link of a dependency chain then costs a look, not a round: rMat
+// 2^24's last nine rounds 89 -> 23 us (with WQ: 1.062 -> 0.943 ms); torus 50^3 78 ->
+// 38 us; randLocal 200,001, whose chains
+// run along the ids, 1.28 -> 0.40 ms; rMat 2^11 42 -> 27 us.
+__device__ __forceinline__ bool wait_out(const MisArgs& a, uint32_t v, uint32_t j, uint32_t e, bool have,
+                                         unsigned long long& in_count) {
+  const int lane = threadIdx.x & 31;
+  bool pending = have;
+  uint32_t cur = j, waits_for = PBG_NONE;  // not walked yet
+  const unsigned long long t0 = dev::globaltimer();
+  for (uint32_t it = 1; __any_sync(FULL, pending); it++) {
+    uint8_t res = UNDECIDED;
+    bool walk = false;
+    if (pending) {
+      if (waits_for == PBG_NONE) {
+        walk = true;
+      } else {
+        const uint8_t f = ld_flag_fresh(a.flags + waits_for);
+        if (f == IN_SET) {
+          res = OUT_SET;
+        } else if (f == OUT_SET) {
+          cur++;
+          walk = true;
+        }
+      }
+    }
+    if (walk) res = walk_lane<LANE_SHARE_LATER, MK_LATER>(a, v, cur, e, &cur);
+    for (unsigned lm = __ballot_sync(FULL, res == MORE); lm; lm &= lm - 1) {
+      const int l = __ffs(lm) - 1;
+      const uint32_t lv = __shfl_sync(FULL, v, l), lj = __shfl_sync(FULL, cur, l), le = __shfl_sync(FULL, e, l);
+      uint32_t lc = lj;
+      const uint8_t r = walk_warp(a, lv, lj, le, &lc);
+      if (lane == l) {
+        res = r;
+        cur = lc;
+      }
+    }
+    if (walk && res == UNDECIDED) waits_for = __ldg(a.edges + cur);  // as read: perhaps decided by now
+    if (pending && res != UNDECIDED) {
+      a.flags[v] = res;
+      if (res == IN_SET) in_count++;
+      pending = false;
+    }
+    if ((it & 255) == 0) {
+      if (dev::ld_acquire_u32(&a.ctrl->sync.error) != 0) return false;
+      if (dev::globaltimer() - t0 > dev::BARRIER_TIMEOUT_NS) {
+        if (lane == 0) atomicOr(&a.ctrl->sync.error, ERR_BARRIER_TIMEOUT);
+        return false;
+      }
+    }
+  }
+  return true;
+}
+
 // Two blocks per SM at <= 40 registers (no spills): 48 resident warps a SM
 // instead of 32 hide more of each walk's load latency (11% on rMat 2^24
 // against one 1024-thread block; 1024 x 2 at 32 registers spills and 512 x 3
@@ -242,7 +313,11 @@ __global__ void __launch_bounds__(BLOCK, 2) mis_persistent(MisArgs a) {
   {
     const unsigned long long tid = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
     const unsigned long long nth = (unsigned long long)gridDim.x * blockDim.x;
-    for (unsigned long long v = tid; v < a.n; v += nth) a.flags[v] = UNDECIDED;
+    const uint32_t mis = (uint32_t)((16 - (reinterpret_cast<uintptr_t>(a.flags) & 15)) & 15);
+    const uint32_t head = min(a.n, mis), n16 = (a.n - head) / 16;
+    uint4* f16 = reinterpret_cast<uint4*>(a.flags + head);
+    for (unsigned long long v = tid; v < n16; v += nth) f16[v] = make_uint4(0, 0, 0, 0);
+    for (unsigned long long v = tid; v < a.n - 16 * n16; v += nth) a.flags[v < head ? v : v + 16 * n16] = UNDECIDED;
     if (tid == 0)
       for (int s = 0; s < 3; s++) c->slot[s] = LevelSlot{0, 0, 0, 0};
   }
@@ -266,6 +341,27 @@ __global__ void __launch_bounds__(BLOCK, 2) mis_persistent(MisArgs a) {
     uint2* cout_ = (r & 1) ? a.c0 : a.c1;
     if (blockIdx.x == 0 && threadIdx.x == 0) c->slot[(r + 2) % 3] = LevelSlot{0, 0, 0, 0};
     const unsigned long long tiles = (nq + 31) / 32;
+    if (tiles <= tw) {  // a lane for every undecided vertex
+      const unsigned long long idx = (unsigned long long)gw * 32 + lane;
+      const bool have = idx < nq;
+      uint32_t v = 0, j = 0, e = 0;
+      if (have) {
+        if (r == 0) {
+          v = (uint32_t)idx;
+          j = __ldg(a.offsets + v);
+          e = __ldg(a.offsets + v + 1);
+        } else {
+          v = qin[idx];
+          const uint2 ce = cin[idx];
+          j = ce.x;
+          e = ce.y;
+        }
+      }
+      wait_out(a, v, j, e, have, in_count);
+      r++;
+      ok = dev::grid_barrier(&c->sync, ERR_BARRIER_TIMEOUT, bar_epoch);
+      break;
+    }
     uint32_t nbuf = 0;
     for (unsigned long long t = gw; t < tiles; t += tw) {
       const unsigned long long idx = t * 32 + lane;
