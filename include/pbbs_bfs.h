@@ -238,11 +238,11 @@ int pbg_bfs_noalloc(const uint32_t* d_offsets, const uint32_t* d_edges, uint32_t
  * 2 = not).  The set is the one serialMIS returns
  * (maximalIndependentSet/serialMIS/MIS.C:33-47: vertices in id order, v in
  * unless an out-neighbour already in the set, a self loop keeping v out),
- * found in parallel rounds on the device and bit-exact with it; on
+ * found in parallel on the device and bit-exact with it; on
  * symmetric graphs it passes MISCheck (bench/MISCheck.C:39-66), the contract
  * of the nondeterministic ndMIS too.  Runs on any graph handle. */
 typedef struct pbg_mis_stats {
-  uint32_t rounds;   /* rounds of the persistent kernel (one grid barrier each) */
+  uint32_t rounds;   /* passes over the vertices (1) */
   uint32_t error;    /* device error word (0 = none) */
   uint64_t in_set;   /* vertices in the set */
   float device_ms;   /* device time of the last call (events) */
@@ -256,9 +256,9 @@ int pbg_mis(pbg_graph* g, uint8_t* flags_out, pbg_mis_stats* stats);
  * synchronised. */
 int pbg_mis_device(pbg_graph* g, uint8_t* d_flags, void* stream);
 int pbg_mis_stats_get(pbg_graph* g, pbg_mis_stats* stats);
-/* Per-round trace of the last MIS on the handle (first PBG_TRACE_LEVELS
- * rounds): `frontier` = the undecided vertices the round walked (n in round
- * 0), `ms` = the round's device time; bottom_up and frontier_degree are 0.
+/* Trace of the last MIS on the handle, one entry per pass: `frontier` = the
+ * vertices it walked (n), `ms` = its device time; bottom_up and
+ * frontier_degree are 0.
  * The reference's timers (common/time_loop.h) time whole calls only.  Call
  * after the stream is synchronised. */
 int pbg_mis_trace(pbg_graph* g, pbg_level_trace* out, uint32_t cap, uint32_t* count);
