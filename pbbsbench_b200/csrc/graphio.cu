@@ -313,23 +313,24 @@ int parse_body(const uint8_t* d_text, uint64_t len, uint64_t n64, uint64_t m64, 
   if (m64 > 0xFFFFFFFFull) return fail(PBG_ERR_ARG, "bad input: m must fit in 32 bits");
   const uint32_t n = (uint32_t)n64;
   const uint64_t nblk = (len + TX_BLOCK - 1) / TX_BLOCK;
-  DevMem cnt, base, err, tmp;
-  unsigned long long total = 0;
+  DevMem scratch;  // block counts, their scan, the scan's scratch, the error word
+  unsigned long long *cnt = nullptr, *base = nullptr, total = 0;
+  size_t tb = 0;
+  const size_t words = (size_t)nblk + 32;
+  if (nblk)
+    PBG_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb, cnt, base, (int64_t)nblk, s));
+  PBG_CUDA(scratch.alloc(2 * sizeof(unsigned long long) * words + tb + 16));
+  unsigned* err = scratch.as<unsigned>();
+  cnt = scratch.as<unsigned long long>() + 32;
+  base = cnt + words - 32;
+  void* tmp = reinterpret_cast<void*>((reinterpret_cast<uintptr_t>(base + nblk) + 15) & ~(uintptr_t)15);
   if (nblk) {
-    PBG_CUDA(cnt.alloc(sizeof(unsigned long long) * nblk));
-    PBG_CUDA(base.alloc(sizeof(unsigned long long) * nblk));
-    k_count_tokens<<<(unsigned)nblk, TX_THREADS, 0, s>>>(d_text, len, cnt.as<unsigned long long>());
+    k_count_tokens<<<(unsigned)nblk, TX_THREADS, 0, s>>>(d_text, len, cnt);
     PBG_CUDA(cudaGetLastError());
-    size_t tb = 0;
-    PBG_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb, cnt.as<unsigned long long>(), base.as<unsigned long long>(),
-                                           (int64_t)nblk, s));
-    PBG_CUDA(tmp.alloc(tb));
-    PBG_CUDA(cub::DeviceScan::ExclusiveSum(tmp.p, tb, cnt.as<unsigned long long>(), base.as<unsigned long long>(),
-                                           (int64_t)nblk, s));
+    PBG_CUDA(cub::DeviceScan::ExclusiveSum(tmp, tb, cnt, base, (int64_t)nblk, s));
     unsigned long long last[2] = {0, 0};
-    PBG_CUDA(cudaMemcpyAsync(&last[0], base.as<unsigned long long>() + nblk - 1, sizeof(last[0]),
-                             cudaMemcpyDeviceToHost, s));
-    PBG_CUDA(cudaMemcpyAsync(&last[1], cnt.as<unsigned long long>() + nblk - 1, sizeof(last[1]),
+    PBG_CUDA(cudaMemcpyAsync(&last[0], base + nblk - 1, sizeof(last[0]), cudaMemcpyDeviceToHost, s));
+    PBG_CUDA(cudaMemcpyAsync(&last[1], cnt + nblk - 1, sizeof(last[1]),
                              cudaMemcpyDeviceToHost, s));
     PBG_CUDA(cudaStreamSynchronize(s));
     total = last[0] + last[1];
@@ -343,18 +344,17 @@ int parse_body(const uint8_t* d_text, uint64_t len, uint64_t n64, uint64_t m64, 
   if (rc) return rc;
   unsigned h_err = 0;
   const uint32_t m32 = (uint32_t)m64;
-  cudaError_t e = err.alloc(sizeof(unsigned));
-  if (e == cudaSuccess) e = cudaMemsetAsync(err.p, 0, sizeof(unsigned), g->stream);
+  cudaError_t e = cudaMemsetAsync(err, 0, sizeof(unsigned), g->stream);
   // the handle's stream runs after the counting pass on s
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e == cudaSuccess && nblk) {
-    k_parse_tokens<<<(unsigned)nblk, TX_THREADS, 0, g->stream>>>(d_text, len, base.as<unsigned long long>(), n, m64,
-                                                               g->d_offsets, g->d_edges, err.as<unsigned>());
+    k_parse_tokens<<<(unsigned)nblk, TX_THREADS, 0, g->stream>>>(d_text, len, base, n, m64, g->d_offsets,
+                                                               g->d_edges, err);
     e = cudaGetLastError();
   }
   if (e == cudaSuccess)  // offsets[n] = m: the tag of common/graphIO.h:207-209
     e = cudaMemcpyAsync(g->d_offsets + n, &m32, sizeof(uint32_t), cudaMemcpyHostToDevice, g->stream);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&h_err, err.p, sizeof(unsigned), cudaMemcpyDeviceToHost, g->stream);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&h_err, err, sizeof(unsigned), cudaMemcpyDeviceToHost, g->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
   if (e != cudaSuccess) {
     pbg_graph_free(g);
