@@ -574,10 +574,13 @@ extern "C" int pbg_graph_upload_device(const uint32_t* d_offsets, const uint32_t
   pbg_graph* g = nullptr;
   int rc = new_handle(n, m, flags, &g);
   if (rc) return rc;
+  // on the default stream: after whatever fills the arrays there or on a
+  // stream that it waits for (the handle's own stream waits for none)
   cudaError_t e = cudaMemcpyAsync(g->d_offsets, d_offsets, sizeof(uint32_t) * ((uint64_t)n + 1),
-                                  cudaMemcpyDeviceToDevice, g->stream);
+                                  cudaMemcpyDeviceToDevice, cudaStreamLegacy);
   if (e == cudaSuccess && m)
-    e = cudaMemcpyAsync(g->d_edges, d_edges, sizeof(uint32_t) * m, cudaMemcpyDeviceToDevice, g->stream);
+    e = cudaMemcpyAsync(g->d_edges, d_edges, sizeof(uint32_t) * m, cudaMemcpyDeviceToDevice, cudaStreamLegacy);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
   if (e != cudaSuccess) {
     pbg_graph_free(g);
     return cuda_fail(e, "graph upload");
