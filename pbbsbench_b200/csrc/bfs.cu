@@ -910,20 +910,14 @@ constexpr uint32_t SMALL_PAD = 64;  // words past the starts that are read, neve
 constexpr uint16_t NO_LEVEL = 0xFFFF;
 
 // Where the line lies: one SM walks 2-4 edges a ns, so levels of many edges
-// are the grid's (SMALL_M), and it probes for many unvisited vertices one
-// after another (SMALL_N).  Bottom-up levels reread the lists that no probe
-// ends early: they stay short where the average list is (SHORT), or where
-// hubs, SKEW times the average, are soon met.  Grid / one block, us a search:
-// rMat 2^10, 8n 44.6 / 21.7; 2^12, 16n 53.0 / 29.7; 2^12, 30n 49.2 / 45.6;
-// torus 11^3 90 / 78, 17^3 131 / 132 (MAX 145 / 130); randLocal 5101, 3 edges
-// within 60 420 / 131; directed 5101, 61 k edges 70.3 / 70.0, 121 k 129 / 103.
-// Past the line: rMat 2^14, 16n 53 / 71; torus 25^3 207 / 337; randLocal 2001,
-// 8 edges 171 / 222; 5101, 20 edges 81 / 120; directed 16001, 192 k 111 / 189.
-constexpr uint64_t SHORT = 8, SKEW = 16;
-bool small_graph(const pbg_graph* g) {
-  if (g->n > SMALL_N || g->m > SMALL_M) return false;
-  return !(g->flags & PBG_GRAPH_SYMMETRIC) || g->m <= SHORT * g->n || (uint64_t)g->max_degree * g->n >= SKEW * g->m;
-}
+// are the grid's (SMALL_M), and so are levels that probe for many unvisited
+// vertices (SMALL_N).  Grid / one block, us a search: rMat 2^10, 8n 44.6 / 22.3;
+// 2^12, 16n 53.0 / 29.7; 2^12, 30n 49.2 / 31.8; torus 17^3 131 / 73; randLocal
+// 5101, 3 edges within 60 420 / 130, 8 within 700 69.6 / 58.3, 20 within 700
+// 81.6 / 70.2, 25 within 100 257 / 162; directed 5101, 61 k edges 70.9 / 70.3,
+// 121 k 125 / 104.  Past the line: randLocal 8001, 8 edges within 1000 76 / 94;
+// rMat 2^13, 14n 53 / 52; directed 8001, 96 k edges 97 / 103.
+bool small_graph(const pbg_graph* g) { return g->n <= SMALL_N && g->m <= SMALL_M; }
 
 size_t small_bytes(uint32_t n, uint32_t nwords) {
   // parents, queue; bitmaps; starts, list begins and vertices of a queue chunk; levels
@@ -1202,7 +1196,14 @@ __global__ void __launch_bounds__(SMALL_T, 1) bfs_small(BfsArgs a) {
         tdl++;
       }
     }
-    if (bu) {
+    // A level that the switch takes bottom-up while its frontier holds few of
+    // the edges is found from the frontier's side all the same: the vertices and
+    // parents are the same, and unvisited vertices that probe in vain for a
+    // frontier of a few dozen cost one SM 18-43 us on rMat 2^12 (5-12 k frontier
+    // edges of 97 k), the frontier's edges 4-6 us; level with each other at a
+    // quarter.
+    const bool few = a.policy == PBG_DIR_AUTO && 4ull * fdeg <= a.m;
+    if (bu && !few) {
       small_bottom_up<MODE>(a, s, L + 1);
     } else {
       for (uint32_t c0 = 0; c0 < nf; c0 += SMALL_T) {
