@@ -30,10 +30,9 @@
 // Parent rules:
 //   ANY: claim by atomicOr on bm[cur] in place; the winner writes parent.
 //   MIN/MAX: every frontier edge into a vertex not in bm[cur] (read-only this
-//     level) does atomicMin/atomicMax on parent; the one that finds it unset
-//     enqueues v and sets its bit in bm[cur^1], which holds level <= L-1 and
-//     receives the frontier's own bits from the threads expanding it; then
-//     cur flips.
+//     level) does atomicMin/atomicMax on parent; the claim that decides who
+//     enqueues v goes to bm[cur^1], which holds level <= L-1 and receives the
+//     frontier's own bits from the threads expanding it; then cur flips.
 //   Bottom-up scans N(v) ascending (MAX: descending) and stops at the first
 //   frontier neighbour, which is the min (max) because lists are sorted.
 //
@@ -230,12 +229,14 @@ __device__ __forceinline__ void emit_k(const BfsArgs& a, const Level& lv, const 
 // running one after another.  Returns the bits of the candidates this lane
 // enqueues.
 // MIN/MAX test the read-only snapshot of the level's visited set first and
-// load ranges for the unvisited only; the reduction that finds the parent
-// unset is the claim.  Large levels are bound by the L1's rate of about one
-// request a clock and SM, and most of their edges lead to visited vertices:
-// a directed graph of 2 M vertices (22.8 M edges reached, MAX) took 0.592 ms
-// with ranges for every edge and a second atomic for every unvisited one,
-// 0.557 ms with these and the arguments selected late (Level).
+// load ranges for the unvisited only: large levels are bound by the L1's rate
+// of about one request a clock and SM, and most of their edges lead to visited
+// vertices.  The claim on the bitmap is issued before the reduction on the
+// parent, which nothing waits for.  us a search, before and now: directed 2 M
+// vertices (22.8 M edges, MAX) 613 / 506, 4 M (MIN) 1486 / 1177, 20 k 129 /
+// 114; torus 100^3 (MIN) 993 / 928.  Letting the reduction that finds the parent
+// unset be the claim saves an atomic, but waits for a word of a large array
+// instead of the bitmap's: 555, 1151, 147, 1179.
 template <int MODE, int K>
 __device__ __forceinline__ unsigned td_claim_k(const BfsArgs& a, const Level& lv, uint32_t u,
                                                const uint32_t (&v)[K], unsigned act, uint32_t (&ob)[K],
@@ -262,19 +263,20 @@ __device__ __forceinline__ unsigned td_claim_k(const BfsArgs& a, const Level& lv
       if ((w[i] >> (v[i] & 31)) & 1u) live &= ~(1u << i);
     load_ranges(a, v, live, ob, oe);
 #pragma unroll
-    for (int i = 0; i < K; i++) {
-      old[i] = 0;
-      if ((live >> i) & 1u)
-        old[i] = (MODE == MODE_MIN) ? atomicMin(a.parent + v[i], u)
-                                    : (uint32_t)atomicMax(reinterpret_cast<int*>(a.parent) + v[i], (int)u);
-    }
+    for (int i = 0; i < K; i++)
+      old[i] = ((live >> i) & 1u) ? atomicOr(lv.claim<MODE>(a) + (v[i] >> 5), 1u << (v[i] & 31)) : FULL;
 #pragma unroll
     for (int i = 0; i < K; i++) {
-      if (old[i] == PBG_NONE) {
-        win |= 1u << i;
-        atomicOr(lv.claim<MODE>(a) + (v[i] >> 5), 1u << (v[i] & 31));
+      if ((live >> i) & 1u) {
+        if (MODE == MODE_MIN)
+          atomicMin(a.parent + v[i], u);
+        else
+          atomicMax(reinterpret_cast<int*>(a.parent) + v[i], (int)u);
       }
     }
+#pragma unroll
+    for (int i = 0; i < K; i++)
+      if (!((old[i] >> (v[i] & 31)) & 1u)) win |= 1u << i;
   }
   if (a.level && win) {
 #pragma unroll
