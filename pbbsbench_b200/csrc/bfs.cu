@@ -134,8 +134,8 @@ __device__ __forceinline__ void load_ranges(const BfsArgs& a, const uint32_t (&v
 // the pointers are selected from the launch arguments where they are used,
 // which costs a select each and keeps some 20 registers free for the loops.
 // The 1024-thread kernels are held to 64 registers: with this and 32-bit
-// per-thread sums they spill 136-156 bytes (bfs_lean 48-72) instead of
-// 184-204 (60-88); torus 160^3 1.677 -> 1.622 ms, rMat 2^24 0.562 -> 0.547 ms,
+// per-thread sums they spill 136-140 bytes (bfs_lean 72) instead of 244-280
+// (196-240); torus 160^3 1.677 -> 1.622 ms, rMat 2^24 0.562 -> 0.547 ms,
 // rMat 2^12 53.2 -> 51.2 us.
 struct Level {
   uint32_t bits;  // 0: output queues are q0/qr0/qb0 (else q1/qr1/qb1); 1: bm1 is the visited bitmap
