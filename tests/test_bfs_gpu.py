@@ -372,3 +372,26 @@ def test_one_block_search_edge_limit(cuda_device):
                 assert np.array_equal(lv, O.bfs_levels(off, edg, 5))
                 assert np.array_equal(par.view(np.uint32), O.bfs_det_parent(off, edg, 5, rule))
         dg.close()
+
+
+@pytest.mark.parametrize("n", [786_431, 786_432, 1_572_863, 2_100_001, 5_000_011])
+def test_host_results_by_either_copy(cuda_device, n):
+    """Host results on both sides of the size from which they go through the pinned ring (6 MiB: one array or two), with
+    one piece more or less and more pieces than the ring holds, to fresh, used and pinned memory: all equal the device's."""
+    import torch
+
+    dg = pb.randlocal_graph(n, 2, max(16, n // 30), 7)
+    d_par = torch.empty(n, dtype=torch.int32, device="cuda")
+    d_lev = torch.empty(n, dtype=torch.int32, device="cuda")
+    dg.bfs_device(3, d_par, d_lev, parent_mode=pb.PARENT_MIN)
+    torch.cuda.synchronize()
+    par0, lev0 = d_par.cpu().numpy(), d_lev.cpu().numpy()
+    for levels in (False, True, True):
+        par, lev, _ = dg.bfs(3, parent_mode=pb.PARENT_MIN, levels=levels)
+        assert np.array_equal(par, par0) and (lev is None or np.array_equal(lev.view(np.int32), lev0))
+    opts = pb.default_opts(parent_mode=pb.PARENT_MIN)
+    pinned = torch.empty(n, dtype=torch.int32, pin_memory=True)
+    plain = np.full(n, -7, np.int32)
+    pb.check(pb.lib().pbg_bfs(dg.handle, 3, ctypes.byref(opts), pinned.data_ptr(), plain.ctypes.data, None))
+    assert np.array_equal(pinned.numpy(), par0) and np.array_equal(plain, lev0)
+    dg.close()

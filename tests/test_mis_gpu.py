@@ -200,3 +200,27 @@ def test_dropin_behind_reference_driver_and_checker(cuda_device, tmp_path):
     c = subprocess.run([CHECKER, gfile, ofile], capture_output=True, text=True, timeout=120)
     assert c.returncode == 0 and c.stdout.strip() == "", c.stdout
     assert np.array_equal(O.read_sequence_int(ofile).astype(np.uint8), O.mis_serial(off, edg))
+
+
+@pytest.mark.parametrize("n", [31, 33, 1000, 227_327, 227_329, 500_003])
+@pytest.mark.parametrize("kind", ["path", "near", "skewed"])
+def test_one_pass_windows(cuda_device, kind, n):
+    """Vertex counts around a tile and around what the grid holds at once (32 vertices for each of 148 x 2 x 24 warps),
+    with chains along the ids (each vertex waits for the one before), short-range edges, and hubs at low and high ids
+    whose lists are walked by the whole warp."""
+    rng = np.random.default_rng(n)
+    i = np.arange(n - 1)
+    if kind == "path":
+        us, vs = i, i + 1
+    elif kind == "near":
+        us = rng.integers(0, n, 4 * n)
+        vs = np.minimum(us + 1 + rng.integers(0, max(1, n // 50), 4 * n), n - 1)
+    else:
+        us = np.concatenate([np.zeros(n // 2, np.int64), np.full(n // 3, n - 1), rng.integers(0, n, 2 * n)])
+        vs = np.concatenate([rng.integers(0, n, n // 2 + n // 3), (rng.random(2 * n) ** 4 * n).astype(np.int64)])
+    keep = us != vs
+    off, edg = O.csr_symmetric(n, us[keep].astype(np.uint32), vs[keep].astype(np.uint32))
+    dg = pb.DeviceGraph.upload(off, edg)
+    for _ in range(2):
+        check_graph(dg, off, edg)
+    dg.close()
