@@ -208,7 +208,9 @@ __device__ __forceinline__ bool settle(const MisArgs& a, uint32_t v, uint32_t j,
       pending = false;
     }
     if ((it & 255) == 0) {  // bounded while nothing moves anywhere
-      if (dev::ld_acquire_u32(&a.ctrl->sync.error) != 0) return false;
+      // a vote: another warp may set the word between two lanes' loads, and
+      // the collectives here and after the pass need every lane
+      if (__any_sync(FULL, dev::ld_acquire_u32(&a.ctrl->sync.error) != 0)) return false;
       const unsigned long long now = dev::globaltimer();
       if (it == 256) {
         t0 = now;
@@ -384,7 +386,7 @@ int mis_read_stats(pbg_graph* g, pbg_mis_stats* st) {
     g->mis_pending = false;
   }
   if (st) *st = g->mis_last;
-  if (g->mis_last.error & ERR_BARRIER_TIMEOUT) return fail(PBG_ERR_TIMEOUT, "MIS: a grid barrier wait ran out");
+  if (g->mis_last.error & ERR_BARRIER_TIMEOUT) return fail(PBG_ERR_TIMEOUT, "MIS: a wait for a neighbour's decision ran out");
   if (g->mis_last.error) return fail(PBG_ERR_STATE, "MIS: device error word set");
   return PBG_OK;
 }
