@@ -66,7 +66,7 @@ struct MisArgs {
   const uint32_t* __restrict__ edges;
   uint8_t* flags;  // UNDECIDED at the start
   BfsCtrl* ctrl;
-  uint32_t* done;  // per warp of the grid: its last finished tile
+  uint32_t* done;  // per warp of the grid: its last finished tile + 1 (0 at the start)
   uint32_t n;
   uint32_t sorted;
 };
@@ -155,7 +155,8 @@ __device__ __forceinline__ uint8_t walk_warp(const MisArgs& a, uint32_t v, uint3
 }
 
 // Whether any warp has finished a tile since *seen was taken (then updated):
-// the order-free sum of the warps' last finished tiles.  Whole warp.
+// the order-free sum of the warps' words, which start at 0 and grow with every
+// tile.  Whole warp.
 __device__ bool progressed(const MisArgs& a, uint32_t warps, uint32_t* seen) {
   uint32_t s = 0;
   for (uint32_t i = threadIdx.x & 31; i < warps; i += 32) s += *reinterpret_cast<volatile uint32_t*>(a.done + i);
@@ -256,7 +257,7 @@ __global__ void __launch_bounds__(BLOCK, 2) mis_one_pass(MisArgs a) {
       ne = __ldg(a.offsets + v + 32 * tw + 1);
     }
     if (!settle(a, v, b, e, v < a.n, tw, in_count)) break;
-    if (lane == 0) *reinterpret_cast<volatile uint32_t*>(a.done + gw) = t;
+    if (lane == 0) *reinterpret_cast<volatile uint32_t*>(a.done + gw) = t + 1;
     b = nb;
     e = ne;
   }
@@ -337,9 +338,10 @@ int mis_launch(pbg_graph* g, uint8_t* d_flags, cudaStream_t s) {
   int grid = 0;
   rc = mis_grid(g->num_sms, &grid);
   if (rc) return rc;
+  const size_t ctrl_bytes = sizeof(BfsCtrl) + sizeof(uint32_t) * (size_t)grid * (MIS_BLOCK / 32);
   if (!g->mis_ctrl) {
     // the control block, then the warps' progress words
-    cudaError_t e = cudaMalloc(&g->mis_ctrl, sizeof(BfsCtrl) + sizeof(uint32_t) * (size_t)grid * (MIS_BLOCK / 32));
+    cudaError_t e = cudaMalloc(&g->mis_ctrl, ctrl_bytes);
     if (e == cudaSuccess && !g->mis_ev0) e = cudaEventCreate(&g->mis_ev0);
     if (e == cudaSuccess && !g->mis_ev1) e = cudaEventCreate(&g->mis_ev1);
     if (e != cudaSuccess) {
@@ -359,7 +361,7 @@ int mis_launch(pbg_graph* g, uint8_t* d_flags, cudaStream_t s) {
   a.n = g->n;
   a.sorted = sorted;
   PBG_CUDA(cudaEventRecord(g->mis_ev0, s));
-  PBG_CUDA(cudaMemsetAsync(g->mis_ctrl, 0, sizeof(BfsCtrl), s));
+  PBG_CUDA(cudaMemsetAsync(g->mis_ctrl, 0, ctrl_bytes, s));
   PBG_CUDA(cudaMemsetAsync(d_flags, UNDECIDED, g->n, s));
   void* params[] = {&a};
   PBG_CUDA(cudaLaunchCooperativeKernel((const void*)mis_one_pass<MIS_BLOCK>, dim3(blocks), dim3(MIS_BLOCK), params,

@@ -64,3 +64,28 @@ def test_a_set_error_word_ends_every_wait(native, n):
     want = O.mis_serial(off, edg)
     assert (got == 0).any() and (got != 0).any()
     assert np.array_equal(got[got != 0], want[got != 0])
+
+
+@pytest.mark.parametrize("n", [31, 1000, 227_329, 500_003])
+@pytest.mark.parametrize("stale", [0, 0xFF])
+def test_every_call_shows_its_own_progress(native, n, stale):
+    """A warp's progress word tells how far it is in this call, whatever the
+    words held before: a finished tile always changes it, also where a warp
+    has one tile and did the same one in the call before."""
+    import torch
+
+    off, edg = path_graph(n)
+    d = on_device(off, edg)
+    flags = torch.empty(n, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    done = np.full(1 << 16, 7, np.uint32)
+    words = ctypes.c_uint32()
+    assert native.mis_progress_words(*args(d, n, len(edg), flags), ctypes.c_int(stale),
+                                     done.ctypes.data_as(ctypes.c_void_p), ctypes.byref(words)) == 0
+    assert np.array_equal(flags.cpu().numpy(), O.mis_serial(off, edg))
+    tiles = (n + 31) // 32
+    warps = min(words.value // 24, tiles) * 24  # 24 warps a block, as many blocks as there are tiles at most
+    last = np.arange(warps) + (np.maximum(tiles - 1 - np.arange(warps), 0) // warps) * warps
+    want = np.zeros(words.value, np.uint32)
+    want[:warps] = np.where(np.arange(warps) < tiles, last + 1, 0)
+    assert np.array_equal(done[: words.value], want)
