@@ -103,9 +103,8 @@ __global__ void check_tails(const uint4* __restrict__ chunks, uint32_t nchunks, 
     bool adj = false;
 #pragma unroll
     for (uint32_t k = 0; k < MS_PULL_CHUNK / 32; k++) {
-      const uint32_t j = ent.y + k * 32 + lane;
-      if (j < ent.z) {
-        const uint32_t u = edges[j];
+      if (k * 32 + lane < ent.z - ent.y) {  // counted from ent.y: a list may end at 2^32 - 1
+        const uint32_t u = edges[ent.y + k * 32 + lane];
         m = min(m, level[u]);
         adj |= (u == pv);
       }
@@ -166,10 +165,12 @@ __global__ void check_rows(const uint32_t* __restrict__ off, const uint32_t* __r
       const uint32_t pl = __shfl_sync(FULL, pv, l);
       uint32_t m2 = n;
       bool a2 = false;
-      for (uint32_t j = bb + lane; j < ee; j += 32) {
-        const uint32_t u = edges[j];
-        m2 = min(m2, L.at(r, u));
-        a2 |= (u == pl);
+      for (uint32_t k = 0; k < ee - bb; k += 32) {  // counted from bb: a list may end at 2^32 - 1
+        if (k + lane < ee - bb) {
+          const uint32_t u = edges[bb + k + lane];
+          m2 = min(m2, L.at(r, u));
+          a2 |= (u == pl);
+        }
       }
       m2 = __reduce_min_sync(FULL, m2);
       a2 = __any_sync(FULL, a2);
@@ -278,16 +279,19 @@ __device__ __forceinline__ uint32_t want_of(uint32_t lv) {
   return __vsub4(lv, 0x01010101u) | none;
 }
 
-// Minimum strip words over the neighbours j, j + step, ... < e.
+// Minimum strip words over the neighbours j, j + step, ... < e (j < e).  What
+// is left of the list is compared, not j + step: e may be 2^32 - 1.
 template <int W, int LPV>
 __device__ __forceinline__ void strip_min(const uint32_t* __restrict__ edges, const uint8_t* __restrict__ strips,
                                           uint32_t part, uint32_t j, uint32_t e, uint32_t step, Words<W>& mn) {
   constexpr uint32_t S = 4 * W * LPV;
   constexpr int K = 4;  // gathers in flight a lane
-  for (; j < e; j += K * step) {
+  for (;; j += K * step) {
+    const uint32_t left = e - j;
+    const uint32_t* p = edges + j;
     uint32_t u[K];
 #pragma unroll
-    for (int k = 0; k < K; k++) u[k] = (j + k * step < e) ? __ldg(edges + j + k * step) : PBG_NONE;
+    for (int k = 0; k < K; k++) u[k] = (k * step < left) ? __ldg(p + k * step) : PBG_NONE;
     Words<W> x[K];
 #pragma unroll
     for (int k = 0; k < K; k++) {
@@ -302,6 +306,7 @@ __device__ __forceinline__ void strip_min(const uint32_t* __restrict__ edges, co
     for (int k = 0; k < K; k++)
 #pragma unroll
       for (int i = 0; i < W; i++) mn.x[i] = __vminu4(mn.x[i], x[k].x[i]);
+    if (left <= K * step) break;
   }
 }
 
@@ -326,7 +331,7 @@ __global__ void strip_tails(const uint4* __restrict__ chunks, uint32_t nchunks, 
     Words<W> mn;
 #pragma unroll
     for (int i = 0; i < W; i++) mn.x[i] = 0xFFFFFFFFu;
-    strip_min<W, LPV>(edges, strips, part, ent.y + grp, ent.z, 32 / LPV, mn);
+    if (grp < ent.z - ent.y) strip_min<W, LPV>(edges, strips, part, ent.y + grp, ent.z, 32 / LPV, mn);
     unsigned long long lo = 0, hi = 0;
 #pragma unroll
     for (int i = 0; i < W; i++) {
@@ -378,7 +383,7 @@ __global__ void __launch_bounds__(256) strip_check(const uint32_t* __restrict__ 
     Words<W> mn;
 #pragma unroll
     for (int i = 0; i < W; i++) mn.x[i] = 0xFFFFFFFFu;
-    strip_min<W, LPV>(edges, strips, part, b, tail ? b + SERIAL : e, 1, mn);
+    if (b < e) strip_min<W, LPV>(edges, strips, part, b, tail ? b + SERIAL : e, 1, mn);
     unsigned long long tl = 0, th = 0;
     if (tail) {
       tl = low[v];

@@ -95,21 +95,21 @@ __device__ __forceinline__ uint8_t ld_flag(const uint8_t* p) {
 // neighbour in an ascending list); MORE with *cur at the first entry not
 // walked when the share is clear and the list goes on.
 __device__ __forceinline__ uint8_t walk_lane(const MisArgs& a, uint32_t v, uint32_t j, uint32_t e, uint32_t* cur) {
-  const uint32_t end = min(e, j + LANE_SHARE);
+  const uint32_t share = min(e - j, LANE_SHARE);  // counted from j: a list may end at 2^32 - 1
   uint32_t first_wait = e;
   bool stop = false;
-  for (; j < end; j += MK) {
+  for (uint32_t k = 0; k < share; k += MK) {
     uint32_t u[MK];
 #pragma unroll
-    for (int i = 0; i < MK; i++) u[i] = (j + i < end) ? __ldg(a.edges + j + i) : v + 1;
+    for (int i = 0; i < MK; i++) u[i] = (k + i < share) ? __ldg(a.edges + j + k + i) : v + 1;
     uint8_t f[MK];
 #pragma unroll
     for (int i = 0; i < MK; i++) f[i] = (u[i] < v) ? ld_flag(a.flags + u[i]) : OUT_SET;
 #pragma unroll
     for (int i = 0; i < MK; i++) {
-      if (j + i >= end) break;
+      if (k + i >= share) break;
       if (u[i] == v || f[i] == IN_SET) return OUT_SET;  // a self loop, or an earlier neighbour in the set
-      if (u[i] < v && f[i] == UNDECIDED && first_wait == e) first_wait = j + i;
+      if (u[i] < v && f[i] == UNDECIDED && first_wait == e) first_wait = j + k + i;
       if (u[i] > v && a.sorted) stop = true;
     }
     // A step with an undecided neighbour ends the walk: the rest of the list
@@ -120,32 +120,35 @@ __device__ __forceinline__ uint8_t walk_lane(const MisArgs& a, uint32_t v, uint3
     *cur = first_wait;
     return UNDECIDED;
   }
-  if (!stop && end < e) {
-    *cur = end;
+  if (!stop && share < e - j) {
+    *cur = j + share;
     return MORE;
   }
   return IN_SET;
 }
 
 // Warp-cooperative walk of one long list (every lane calls it with the same
-// v, j, e).
+// v, j, e; j < e).
 __device__ __forceinline__ uint8_t walk_warp(const MisArgs& a, uint32_t v, uint32_t j, uint32_t e, uint32_t* cur) {
-  const int lane = threadIdx.x & 31;
+  const uint32_t lane = threadIdx.x & 31;
   uint32_t first_wait = e;
-  for (uint32_t j0 = j; j0 < e; j0 += 32) {
-    const uint32_t p = j0 + lane;
+  for (;; j += 32) {
+    const bool have = lane < e - j;
     uint32_t u = v + 1;
     uint8_t f = OUT_SET;
-    if (p < e) {
-      u = __ldg(a.edges + p);
+    if (have) {
+      u = __ldg(a.edges + j + lane);
       if (u < v) f = ld_flag(a.flags + u);
     }
-    const bool out = p < e && (u == v || f == IN_SET);
+    const bool out = have && (u == v || f == IN_SET);
     if (__any_sync(FULL, out)) return OUT_SET;
-    const unsigned w = __ballot_sync(FULL, p < e && u < v && f == UNDECIDED);
-    if (w && first_wait == e) first_wait = j0 + __ffs(w) - 1;
-    if (first_wait < e) break;  // as in walk_lane: resume at the first undecided neighbour
-    if (a.sorted && __any_sync(FULL, p < e && u > v)) break;
+    const unsigned w = __ballot_sync(FULL, have && u < v && f == UNDECIDED);
+    if (w) {  // as in walk_lane: resume at the first undecided neighbour
+      first_wait = j + __ffs(w) - 1;
+      break;
+    }
+    if (a.sorted && __any_sync(FULL, have && u > v)) break;
+    if (e - j <= 32) break;
   }
   if (first_wait < e) {
     *cur = first_wait;
@@ -279,7 +282,7 @@ __global__ void k_lists_sorted(const uint32_t* __restrict__ off, const uint32_t*
   for (uint32_t v = w; v < n; v += nw) {
     const uint32_t b = off[v], e = off[v + 1];
     bool unsorted = false;
-    for (uint32_t j = b + 1 + lane; j < e; j += 32) unsorted |= edg[j - 1] > edg[j];
+    for (uint64_t j = (uint64_t)b + 1 + lane; j < e; j += 32) unsorted |= edg[j - 1] > edg[j];
     if (__any_sync(FULL, unsorted)) {
       if (lane == 0) atomicOr(bad, 1u);
     }

@@ -40,7 +40,7 @@ __global__ void pull_chunk_fill(const uint32_t* __restrict__ off, uint32_t n, co
   const uint32_t s = start[v], c = start[v + 1] - s, b = off[v] + MS_PULL_SERIAL, e = off[v + 1];
   for (uint32_t i = 0; i < c; i++) {
     const uint32_t cb = b + i * MS_PULL_CHUNK;
-    out[s + i] = make_uint4(v, cb, min(e, cb + MS_PULL_CHUNK), e - off[v]);
+    out[s + i] = make_uint4(v, cb, cb + min(e - cb, MS_PULL_CHUNK), e - off[v]);  // e may be 2^32 - 1
   }
 }
 
