@@ -616,9 +616,10 @@ extern "C" int pbg_levels_check(pbg_graph* g, const uint32_t* srcs, uint32_t row
   const size_t kept = g->check_bytes;
   void* sp = nullptr;
   int rc = PBG_OK;
-  if (stride) {
+  if (stride) {  // check_rows needs no table of the list tails: it is what runs where that does not fit
     rc = ms_pull_chunks(g);
-    if (rc) return rc;
+    if (rc && rc != PBG_ERR_OOM) return rc;
+    if (rc) stride = 0;
     for (; stride; stride = stride > 16 ? stride / 2 : stride > 4 ? 4 : 0) {
       rc = check_scratch(g, head + ((16ull * g->n + 255) & ~255ull) + (size_t)stride * g->n, &sp);
       if (rc != PBG_ERR_OOM) break;

@@ -188,3 +188,89 @@ def test_levels_rows_in_strips(cuda_device, n, k):
             bad[r, v] = to if bad[r, v] != to else to ^ 1
             assert both(bad) is not None or n < 255
     dg.close()
+
+
+class _Hog:
+    """Takes all device memory but `left` bytes."""
+
+    def __init__(self, left):
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        free, _ = torch.cuda.mem_get_info()
+        self.block = torch.empty(max(0, free - left) >> 21 << 21, dtype=torch.uint8, device="cuda")
+        now, _ = torch.cuda.mem_get_info()
+        assert abs(now - left) <= 4 << 20, (free, now, left)
+
+    def release(self):
+        self.block = None
+        torch.cuda.empty_cache()
+
+
+@pytest.fixture
+def hog(cuda_device):
+    held = []
+
+    def take(left):
+        held.append(_Hog(left))
+
+    yield take
+    for h in held:
+        h.release()
+
+
+def _warm_levels_check():
+    """Every width's kernels once: a kernel is loaded into device memory when it is first launched."""
+    off, edg = O.csr_symmetric(700, np.zeros(600, np.uint32), np.arange(1, 601, dtype=np.uint32))
+    for cut, ks in ((700, (2, 12, 20, 40)), (200, (2,))):
+        o = np.minimum(off[: cut + 1], 0) if cut < 700 else off
+        dg = pb.DeviceGraph.upload(o, edg[: o[-1]])
+        for k in ks:
+            rows = np.full((k, cut), 255, np.uint8)
+            dg.levels_check(np.zeros(k, np.uint32), torch.from_numpy(rows).cuda())
+        dg.close()
+
+
+def test_level_rows_without_memory_for_the_tail_table(hog):
+    """Lists of 40,000 entries (every neighbour twenty times over): the table of their tails takes 10 MB.  With less
+    than that left the rows are checked all the same."""
+    n, reach, times = 4096, 1000, 20
+    d = torch.arange(1, reach + 1, dtype=torch.int32, device="cuda")
+    to = torch.cat([d, -d]).repeat_interleave(times)
+    edges = (torch.arange(n, dtype=torch.int32, device="cuda")[:, None] + to[None, :]).remainder_(n).reshape(-1)
+    off = torch.arange(n + 1, dtype=torch.int64, device="cuda").mul_(2 * reach * times).to(torch.int32)
+    dg = pb.DeviceGraph.upload(off, edges)
+    del edges, to
+    srcs = np.array([0, 1777], np.uint32)
+    gap = np.abs(np.arange(n)[None, :] - srcs[:, None])
+    rows = (-(-np.minimum(gap, n - gap) // reach)).astype(np.uint8)
+    bad = rows.copy()
+    bad[1, 3000] += 1
+    d_rows, d_bad = torch.from_numpy(rows).cuda(), torch.from_numpy(bad).cuda()
+    _warm_levels_check()
+    hog(6 << 20)
+    assert dg.levels_check(srcs, d_rows)["bad_vertex"] == NONE
+    got = dg.levels_check(srcs, d_bad)
+    assert got["row"] == 1 and got["bad_vertex"] <= 3000
+    dg.close()
+
+
+@pytest.mark.parametrize("left", [250, 150, 100, 40])
+def test_level_rows_in_narrower_strips(hog, left):
+    """40 rows of 4.1 M vertices take 328 MB of scratch in strips of 64; with 250, 150, 100 and 40 MB left they go
+    through strips of 32, 16 and 4 rows, and row by row."""
+    k = 40
+    make = lambda: pb.torus3d_graph(160, perm_seed=3)  # noqa: E731
+    with_levels = make()
+    srcs = np.arange(5, 5 + 1000 * k, 1000, dtype=np.uint32)
+    rows, _ = with_levels.bfs_multi(srcs)
+    with_levels.close()
+    dg = make()
+    d_rows = torch.from_numpy(rows).cuda()
+    v = int(np.argmax(rows[33]))
+    _warm_levels_check()
+    hog(left << 20)
+    assert dg.levels_check(srcs, d_rows)["bad_vertex"] == NONE
+    d_rows[33, v] += 1
+    got = dg.levels_check(srcs, d_rows)
+    assert got["row"] == 33 and got["bad_vertex"] <= v
+    dg.close()
