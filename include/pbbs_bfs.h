@@ -66,7 +66,11 @@ typedef struct pbg_graph pbg_graph;
 int pbg_graph_upload(const uint32_t* offsets, const uint32_t* edges, uint32_t n, uint64_t m,
                      uint32_t flags, pbg_graph** out);
 
-/* Same, from device memory (the arrays are copied). */
+/* Same, from device memory (the arrays are copied).  The copies run on the
+ * default stream: after whatever was enqueued there, or on streams that it
+ * waits for, before the call.  A caller that fills the arrays on a stream made
+ * with cudaStreamNonBlocking, or on a per-thread default stream, waits for it
+ * first.  The arrays may be changed or freed when the call returns. */
 int pbg_graph_upload_device(const uint32_t* d_offsets, const uint32_t* d_edges, uint32_t n,
                             uint64_t m, uint32_t flags, pbg_graph** out);
 

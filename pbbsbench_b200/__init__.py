@@ -82,6 +82,8 @@ class DeviceGraph:
 
     @classmethod
     def upload(cls, offsets, edges, symmetric: bool = True) -> "DeviceGraph":
+        """A resident graph from CSR arrays: numpy arrays, or torch tensors on
+        the device as the current torch stream leaves them."""
         h = ctypes.c_void_p()
         flags = _capi.GRAPH_SYMMETRIC if symmetric else 0
         if isinstance(offsets, np.ndarray):
@@ -92,6 +94,10 @@ class DeviceGraph:
             check(lib().pbg_graph_upload(_ptr(offsets), _ptr(edges), len(offsets) - 1, int(offsets[-1]), flags,
                                          ctypes.byref(h)))
         else:  # torch tensors on the device
+            if offsets.is_cuda:  # what fills them may still be queued on a stream that the copies do not wait for
+                import torch
+
+                torch.cuda.current_stream(offsets.device).synchronize()
             check(lib().pbg_graph_upload_device(_ptr(offsets), _ptr(edges), offsets.numel() - 1, edges.numel(),
                                                 flags, ctypes.byref(h)))
         return cls(h)

@@ -395,3 +395,26 @@ def test_host_results_by_either_copy(cuda_device, n):
     pb.check(pb.lib().pbg_bfs(dg.handle, 3, ctypes.byref(opts), pinned.data_ptr(), plain.ctypes.data, None))
     assert np.array_equal(pinned.numpy(), par0) and np.array_equal(plain, lev0)
     dg.close()
+
+
+@pytest.mark.parametrize("side", [False, True])
+def test_upload_waits_for_the_stream_that_fills_the_arrays(cuda_device, side):
+    """Device arrays whose filling is still queued behind other work when the upload is called, on the default stream
+    and inside a side stream's context: the handle holds what they are filled with."""
+    import contextlib
+
+    import torch
+
+    off, edg = O.torus3d(40, 3)
+    src_off, src_edg = (torch.from_numpy(a.view(np.int32)).cuda() for a in (off, edg))
+    d_off, d_edg = torch.zeros_like(src_off), torch.zeros_like(src_edg)
+    torch.cuda.synchronize()
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream) if side else contextlib.nullcontext():
+        torch.cuda._sleep(200_000_000)  # about a tenth of a second
+        d_off.copy_(src_off)
+        d_edg.copy_(src_edg)
+        dg = pb.DeviceGraph.upload(d_off, d_edg)
+    got = dg.download()
+    assert np.array_equal(got[0], off) and np.array_equal(got[1], edg)
+    dg.close()
