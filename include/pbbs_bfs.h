@@ -167,7 +167,7 @@ typedef struct pbg_bfs_stats {
   uint32_t error;           /* device error word (0 = none) */
   uint64_t visited;         /* reached vertices */
   uint64_t edges_reached;   /* sum of degrees of reached vertices (m_r) */
-  uint64_t bottomup_mask;   /* bit L set: level L (< 64) ran bottom-up (small graphs: was the switch's choice) */
+  uint64_t bottomup_mask;   /* bit L set: level L (< 64) ran bottom-up */
   float device_ms;          /* device time of the last pbg_bfs call (events) */
   float init_ms;            /* of which: kernel start to the first level (initialisation) */
   float kernel_ms;          /* kernel start to end as seen by the device clock */

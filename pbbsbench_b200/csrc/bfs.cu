@@ -1183,29 +1183,30 @@ __global__ void __launch_bounds__(SMALL_T, 1) bfs_small(BfsArgs a) {
       bu = (unsigned long long)nf + fdeg > a.m / a.alpha;
     else
       bu = nf > a.n / a.beta;
+    // A level that the switch takes bottom-up while its frontier holds few of
+    // the edges is found from the frontier's side all the same: the vertices are
+    // the same, and so are MIN and MAX parents, and unvisited vertices that probe
+    // in vain for a frontier of a few dozen cost one SM 18-43 us on rMat 2^12
+    // (5-12 k frontier edges of 97 k), the frontier's edges 4-6 us; level with
+    // each other at a quarter.  The switch goes on from its own choice (bu); what
+    // is reported is what ran.
+    const bool up = bu && !(a.policy == PBG_DIR_AUTO && 4ull * fdeg <= a.m);
     if (tid == 0) {
       if (L < PBG_TRACE_LEVELS) {
         c->t_ns[L] = globaltimer();
         c->t_nf[L] = nf;
         c->t_deg[L] = fdeg;
-        c->t_bu[L] = bu ? 1u : 0u;
+        c->t_bu[L] = up ? 1u : 0u;
       }
       reached += fdeg;
-      if (bu) {
+      if (up) {
         bul++;
         if (L < 64) bumask |= 1ull << L;
       } else {
         tdl++;
       }
     }
-    // A level that the switch takes bottom-up while its frontier holds few of
-    // the edges is found from the frontier's side all the same: the vertices and
-    // parents are the same, and unvisited vertices that probe in vain for a
-    // frontier of a few dozen cost one SM 18-43 us on rMat 2^12 (5-12 k frontier
-    // edges of 97 k), the frontier's edges 4-6 us; level with each other at a
-    // quarter.
-    const bool few = a.policy == PBG_DIR_AUTO && 4ull * fdeg <= a.m;
-    if (bu && !few) {
+    if (up) {
       small_bottom_up<MODE>(a, s, L + 1);
     } else {
       for (uint32_t c0 = 0; c0 < nf; c0 += SMALL_T) {
@@ -1231,7 +1232,7 @@ __global__ void __launch_bounds__(SMALL_T, 1) bfs_small(BfsArgs a) {
       }
     }
     __syncthreads();
-    if (bu || MODE != MODE_ANY) {
+    if (up || MODE != MODE_ANY) {
       for (uint32_t w = tid; w < nw; w += SMALL_T) {
         const uint32_t f = s.fresh[w];
         if (f) {

@@ -418,3 +418,28 @@ def test_upload_waits_for_the_stream_that_fills_the_arrays(cuda_device, side):
     got = dg.download()
     assert np.array_equal(got[0], off) and np.array_equal(got[1], edg)
     dg.close()
+
+
+@pytest.mark.parametrize("kind", ["rmat", "torus", "randlocal"])
+def test_small_graphs_report_the_direction_that_ran(cuda_device, kind):
+    """The one-block search takes a level from the frontier's side when the frontier has at most a quarter of the edges,
+    also where the switch says bottom-up: trace, counts and mask name what ran.  The fixed directions run as asked."""
+    off, edg = {"rmat": lambda: O.rmat(12, 16 << 12, 3, 0.57, 0.19, 0.19), "torus": lambda: O.torus3d(16, 5),
+                "randlocal": lambda: O.randlocal(5000, 8, 700, 4)}[kind]()
+    dg = pb.DeviceGraph.upload(off, edg)
+    few = 0
+    for src in (0, 17, 1234):
+        for mode in MODES:
+            for direction in DIRS:
+                _, st = check_run(dg, off, edg, src, mode, direction)
+                tr = dg.trace()
+                up = [t["dir"] == "bottom-up" for t in tr]
+                if direction == pb.DIR_AUTO:
+                    assert all(4 * t["frontier_degree"] > dg.m for t, b in zip(tr, up) if b)
+                    few += sum(t["frontier"] + t["frontier_degree"] > dg.m // 20 and not b for t, b in zip(tr, up))
+                else:
+                    assert all(b == (direction == pb.DIR_BOTTOMUP) for b in up)
+                assert st["bottomup_levels"] == sum(up) and st["topdown_levels"] == len(up) - sum(up)
+                assert st["bottomup_mask"] == sum(1 << i for i, b in enumerate(up[:64]) if b)
+    assert few  # the switch's bottom-up levels that were taken from the frontier's side
+    dg.close()
