@@ -1510,8 +1510,11 @@ int bfs_launch(pbg_graph* g, uint32_t src, const pbg_bfs_opts& o, uint32_t* d_pa
 }
 
 int bfs_read_trace(pbg_graph* g, pbg_level_trace* out, uint32_t cap, uint32_t* count) {
-  if (!g->ws.ready) return fail(PBG_ERR_STATE, "no BFS has run on this graph");
   int rc = bfs_read_stats(g, nullptr);
+  if (!g->ws.ready) {  // no search: an error, or no levels (bfs_read_stats)
+    if (!rc && count) *count = 0;
+    return rc;
+  }
   if (rc && rc != PBG_ERR_TIMEOUT && rc != PBG_ERR_STATE) return rc;
   BfsCtrl* c = new BfsCtrl;
   cudaError_t e = cudaMemcpy(c, g->ws.ctrl, sizeof(BfsCtrl), cudaMemcpyDeviceToHost);
@@ -1533,8 +1536,10 @@ int bfs_read_trace(pbg_graph* g, pbg_level_trace* out, uint32_t cap, uint32_t* c
   return PBG_OK;
 }
 
+// The last search's statistics; all zero on a handle that so far only ran an
+// independent set.
 int bfs_read_stats(pbg_graph* g, pbg_bfs_stats* st) {
-  if (!g->ws.ready) return fail(PBG_ERR_STATE, "no BFS has run on this graph");
+  if (!g->ws.ready && !g->mis_ran) return fail(PBG_ERR_STATE, "no BFS has run on this graph");
   if (g->stats_pending) {
     BfsCtrl c;
     PBG_CUDA(cudaEventSynchronize(g->ws.ev1));

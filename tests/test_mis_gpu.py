@@ -164,6 +164,20 @@ def test_bfs_statistics_survive_an_mis_call(cuda_device):
     dg.close()
 
 
+def test_search_statistics_of_a_handle_that_only_ran_the_set(cuda_device):
+    """Zeros and an empty trace, as before any search; a handle on which nothing has run has none to give."""
+    off, edg = O.torus3d(12, 1)
+    dg = pb.DeviceGraph.upload(off, edg)
+    with pytest.raises(pb.PbgError, match="no BFS"):
+        dg.last_stats()
+    dg.mis()
+    st = dg.last_stats()
+    assert st["levels"] == 0 and st["visited"] == 0 and st["error"] == 0 and dg.trace() == []
+    dg.bfs(0)
+    assert dg.last_stats()["visited"] == dg.n and len(dg.trace()) > 0
+    dg.close()
+
+
 def test_device_buffers_and_python_entry_point(cuda_device):
     import torch
 
