@@ -215,7 +215,7 @@ def build(verbose: bool = False, jobs: int | None = None) -> str:
     from concurrent.futures import ThreadPoolExecutor
 
     os.makedirs(BUILD_DIR, exist_ok=True)
-    headers = glob.glob(os.path.join(PKG, "csrc", "*.cuh")) + glob.glob(os.path.join(INCLUDE, "*.h"))
+    headers = [h for kind in ("*.cuh", "*.h") for h in glob.glob(os.path.join(PKG, "csrc", kind))] + glob.glob(os.path.join(INCLUDE, "*.h"))
     newest_dep = max([os.path.getmtime(h) for h in headers] + [os.path.getmtime(__file__)])
     jobs_to_run, objs = [], []
     for src in sources():
