@@ -3,15 +3,13 @@
 // A copy to pageable memory goes through the driver's staging on one host
 // thread, which also takes the page faults of a freshly allocated result
 // array: parents and levels of rMat 2^20 (8 MB into new arrays) were 1.7 ms
-// of a 1.8 ms call.  Large results for pageable memory go through a pinned
-// ring here instead: the device copies piece after piece into it and several
-// host threads move each piece on, so the faults are taken in parallel and
-// overlap the link: rMat 2^20 2.0 -> 0.99 ms a call, randLocal 6,000,001 (48 MB
-// of results) 13.2 -> 5.6 ms.  The line (MIN_STAGED): results of 5.6 MB in all
-// mostly go to arrays whose pages the process has already (0.75 ms plain,
-// 1.03 through the ring, whose threads cost 0.1-0.2 ms to start and wake);
-// from about 6.4 MB the allocator maps them anew (3.4 ms plain, 1.3 ms).
-// Pinned destinations get the plain copy, at the link's rate.
+// of a 1.8 ms call.  Results that are large, or whose memory has no pages yet
+// (worth_ring in hostmove.h: the lines and what they measured), go through a
+// pinned ring here instead: the device copies piece after piece into it and
+// several host threads move each piece on, so the faults are taken in parallel
+// and overlap the link: rMat 2^20 into new arrays 2.0 -> 0.99 ms a call,
+// randLocal 6,000,001 (48 MB of results) 13.2 -> 5.6 ms.  Pinned destinations
+// get the plain copy, at the link's rate.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -28,7 +26,6 @@ using hostmove::Moved;
 using hostmove::PIECE;
 using hostmove::Piece;
 using hostmove::RING;
-constexpr size_t MIN_STAGED = 6ull << 20;  // bytes of a call; see above
 
 // The ring is pinned on first use (a few ms) and kept for the process, as the
 // file transfers' pieces are; a call that finds it in use copies plainly.
@@ -91,15 +88,14 @@ struct RingLink {
   }
 };
 
-// The pageable copies' pieces; false when there is no memory for the list.
-bool cut(const HostCopy* copies, int count, std::vector<Piece>* out) {
+// The pieces of the copies marked in `ring`; false when there is no memory for
+// the list.
+bool cut(const HostCopy* copies, int count, const bool* ring, std::vector<Piece>* out) {
   try {
-    for (int i = 0; i < count; i++) {
-      const HostCopy& c = copies[i];
-      if (!c.dst || !pageable(c.dst)) continue;
-      for (size_t o = 0; o < c.bytes; o += PIECE)
-        out->push_back({static_cast<char*>(c.dst) + o, static_cast<const char*>(c.src) + o, std::min(PIECE, c.bytes - o)});
-    }
+    for (int i = 0; i < count; i++)
+      for (size_t o = 0; ring[i] && o < copies[i].bytes; o += PIECE)
+        out->push_back({static_cast<char*>(copies[i].dst) + o, static_cast<const char*>(copies[i].src) + o,
+                        std::min(PIECE, copies[i].bytes - o)});
   } catch (...) {
     return false;
   }
@@ -109,36 +105,42 @@ bool cut(const HostCopy* copies, int count, std::vector<Piece>* out) {
 }  // namespace
 
 int copy_out(const HostCopy* copies, int count, cudaStream_t s) {
+  constexpr int MAX = 2;
+  if (count > MAX) return fail(PBG_ERR_ARG, "copy_out: too many copies");
+  hostmove::Range to[MAX];
+  bool ring[MAX] = {};  // the pageable ones, where the call takes the ring
   size_t total = 0;
+  int nto = 0;
   for (int i = 0; i < count; i++) total += copies[i].dst ? copies[i].bytes : 0;
-  const bool large = total >= MIN_STAGED;
-  auto plain = [&](bool pageables) -> int {
-    for (int i = 0; i < count; i++) {
-      const HostCopy& c = copies[i];
-      if (c.dst && c.bytes && (!large || pageable(c.dst)) == pageables)
-        PBG_CUDA(cudaMemcpyAsync(c.dst, c.src, c.bytes, cudaMemcpyDeviceToHost, s));
-    }
+  for (int i = 0; i < count && total >= hostmove::MIN_RING; i++) {
+    ring[i] = copies[i].dst && copies[i].bytes && pageable(copies[i].dst);
+    if (ring[i]) to[nto++] = {copies[i].dst, copies[i].bytes};
+  }
+  const bool worth = hostmove::worth_ring(to, nto);
+  auto plain = [&](bool want) -> int {
+    for (int i = 0; i < count; i++)
+      if (copies[i].dst && copies[i].bytes && (worth && ring[i]) == want)
+        PBG_CUDA(cudaMemcpyAsync(copies[i].dst, copies[i].src, copies[i].bytes, cudaMemcpyDeviceToHost, s));
     return PBG_OK;
   };
-  bool staged = false;
-  if (large) {
-    const int rc = plain(false);
-    if (rc) return rc;
+  int rc = plain(false);
+  if (rc) return rc;
+  if (worth) {
     std::vector<Piece> pieces;
     std::unique_lock<std::mutex> lk(g_ring.mu, std::defer_lock);
-    if (cut(copies, count, &pieces) && !pieces.empty() && lk.try_lock() && ring_ready(g_ring)) {
+    Moved m = Moved::NOT_BEGUN;
+    if (cut(copies, count, ring, &pieces) && lk.try_lock() && ring_ready(g_ring)) {
       RingLink link{g_ring, s};
-      const Moved m = hostmove::move_pieces(pieces, g_ring.mem, link);
+      m = hostmove::move_pieces(pieces, g_ring.mem, link);
       if (m == Moved::LINK_FAILED) {
         cudaStreamSynchronize(s);  // no copy into the ring is left in flight
         return cuda_fail(link.e, "result copy");
       }
-      staged = m == Moved::ALL;
     }
-  }
-  if (!staged) {
-    const int rc = plain(true);
-    if (rc) return rc;
+    if (m == Moved::NOT_BEGUN) {
+      rc = plain(true);
+      if (rc) return rc;
+    }
   }
   PBG_CUDA(cudaStreamSynchronize(s));
   return PBG_OK;

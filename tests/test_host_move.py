@@ -19,3 +19,10 @@ def test_pieces_through_the_ring(tmp_path):
     exception."""
     r = subprocess.run([_program(tmp_path, "host_move")], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and r.stdout.splitlines()[-1] == "all right", r.stdout + r.stderr
+
+
+def test_which_results_take_the_ring(tmp_path):
+    """Results of 6 to 16 MiB take the ring only when memory for a MiB or more of them is not there yet: a result
+    buffer that is used again goes by plain copies, which are faster at these sizes."""
+    r = subprocess.run([_program(tmp_path, "ring_rule")], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0 and r.stdout.splitlines()[-1] == "all right", r.stdout + r.stderr
