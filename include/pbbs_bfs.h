@@ -50,6 +50,12 @@ typedef struct pbg_graph pbg_graph;
  * call that creates a handle returns PBG_ERR_ARG for a larger n. */
 #define PBG_MAX_VERTICES 0x7FFFFFFFu
 
+/* Largest edge count that the searches take.  A handle holds up to 2^32 - 1
+ * edges (offsets are uint32), and checks and independent sets run on all of
+ * them; the searches' edge positions, 32 bits wide, step up to 64 past a
+ * list's end, so they return PBG_ERR_ARG for a larger m. */
+#define PBG_MAX_SEARCH_EDGES 0xFFFFFFBFu
+
 /* The graph is symmetric (every edge present in both directions).  Only then
  * may BFS run bottom-up, which scans N(v) as in-neighbours exactly as
  * edge_map_dense does (common/ligraLight.h:87-112). */

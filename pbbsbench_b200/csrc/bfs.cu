@@ -293,16 +293,15 @@ __device__ __forceinline__ void td_chunk(const BfsArgs& a, const uint4& ent, uin
   const int lane = threadIdx.x & 31;
   const uint32_t u = ent.x;
   const uint32_t cb = ent.y + c_local * CHUNK;
-  const uint32_t ce = min(ent.z, cb + CHUNK);
+  const uint32_t len = min(ent.z - cb, CHUNK);  // positions counted from cb: a list may end at 2^32 - 1
   if (MODE != MODE_ANY && c_local == 0 && lane == 0) atomicOr(lv.claim<MODE>(a) + (u >> 5), 1u << (u & 31));
   uint32_t v[PER_LANE];
   unsigned act = 0;
 #pragma unroll
   for (int i = 0; i < PER_LANE; i++) {
-    const uint32_t j = cb + i * 32 + lane;
     v[i] = 0;
-    if (j < ce) {
-      v[i] = __ldg(a.edges + j);
+    if (i * 32 + lane < len) {
+      v[i] = __ldg(a.edges + (cb + i * 32 + lane));
       act |= 1u << i;
     }
   }
@@ -443,12 +442,11 @@ __device__ __forceinline__ void bu_word(const BfsArgs& a, const uint32_t* vin, u
         }
       }
     } else {
-      for (uint32_t j0 = bb + LSHARE; j0 < ee && !got; j0 += 32) {
-        const uint32_t j = j0 + lane;
+      for (uint32_t k = LSHARE; k < ee - bb && !got; k += 32) {  // counted from bb: a list may end at 2^32 - 1
         uint32_t x = 0;
         bool h = false;
-        if (j < ee) {
-          x = __ldg(a.edges + j);
+        if (k + lane < ee - bb) {
+          x = __ldg(a.edges + (bb + k + lane));
           h = (vin[x >> 5] >> (x & 31)) & 1u;
         }
         const unsigned hb = __ballot_sync(FULL, h);
@@ -1356,6 +1354,9 @@ void resolve_graph_opts(const pbg_graph* g, const pbg_bfs_opts* in, bool multi, 
     resolve_opts(multi ? &g->tuned_multi : &g->tuned, o);
   else
     resolve_opts(in, o);
+  // the lanes of a tile step together, so a short list's position runs up to
+  // the chunk degree past its end (td_small, lean_tile): not past 2^32
+  if (g && !multi && g->m + o->chunk_min_degree + PER_LANE > (1ull << 32)) o->chunk_min_degree = 32;
 }
 
 int bfs_ensure_workspace(pbg_graph* g, const pbg_bfs_opts& o) {
@@ -1453,6 +1454,7 @@ int bfs_launch(pbg_graph* g, uint32_t src, const pbg_bfs_opts& o, uint32_t* d_pa
   if (o.block_threads != 256 && o.block_threads != 512 && o.block_threads != 1024)
     return fail(PBG_ERR_ARG, "block_threads must be 256, 512 or 1024");
   if (o.chunk_min_degree < 1) return fail(PBG_ERR_ARG, "chunk_min_degree must be >= 1");
+  if (g->m > PBG_MAX_SEARCH_EDGES) return fail(PBG_ERR_ARG, "searches take at most PBG_MAX_SEARCH_EDGES edges");
   int rc = bfs_ensure_workspace(g, o);
   if (rc) return rc;
   BfsWorkspace& w = g->ws;

@@ -449,8 +449,8 @@ __device__ void pull_chunk_group(const MsJob& J, uint32_t group, const unsigned 
     uint32_t u[PCH_STEPS];
 #pragma unroll
     for (int i = 0; i < PCH_STEPS; i++) {
-      const uint32_t j = cb + i * 32 + lane;
-      u[i] = (j < ce) ? __ldg(J.edges + j) : NONE32;
+      // counted from cb: a list may end at 2^32 - 1
+      u[i] = (i * 32 + lane < ce - cb) ? __ldg(J.edges + (cb + i * 32 + lane)) : NONE32;
     }
     Mask<W> acc = mzero<W>();
 #pragma unroll
@@ -651,21 +651,21 @@ __device__ void range_push(const MsJob& J, uint32_t tile, unsigned long long nq,
   __syncwarp();
 }
 
-// Push of one chunk [cb, ce) of a frontier vertex with mask f, by the whole
-// warp, 32 * RUN edges a step.
+// Push of one chunk of a frontier vertex with mask f (`len` edges from cb: the
+// chunk may end at 2^32 - 1), by the whole warp, 32 * RUN edges a step.
 template <int PM, int W>
-__device__ __forceinline__ void chunk_push(const MsJob& J, uint32_t cb, uint32_t ce, const Mask<W>& f,
+__device__ __forceinline__ void chunk_push(const MsJob& J, uint32_t cb, uint32_t len, const Mask<W>& f,
                                            unsigned long long* fnext, LevelSlot* out, uint32_t* qout,
                                            uint4* qbout, uint32_t big_deg, unsigned long long* s_deg) {
   constexpr int RUN = (PM == PM_DENSE && W < 4) ? PCH_STEPS : 4;
   const int lane = threadIdx.x & 31;
-  for (uint32_t j0 = cb; j0 < ce; j0 += 32 * RUN) {
+  for (uint32_t k0 = 0; k0 < len; k0 += 32 * RUN) {
     uint32_t jj[RUN];
     Mask<W> ff[RUN];
 #pragma unroll
     for (int i = 0; i < RUN; i++) {
-      const uint32_t j = j0 + i * 32 + lane;
-      jj[i] = (j < ce) ? j : NONE32;
+      const uint32_t k = k0 + i * 32 + lane;
+      jj[i] = (k < len) ? cb + k : NONE32;
       ff[i] = f;
     }
     if constexpr (PM == PM_SPARSE)
@@ -695,7 +695,7 @@ __device__ void vchunk_push(const MsJob& J, uint32_t group, const unsigned long 
     mm &= mm - 1;
     const uint32_t cb = __shfl_sync(FULL, ent.y, l);
     const uint32_t ce = __shfl_sync(FULL, ent.z, l);
-    chunk_push<PM, W>(J, cb, ce, mshfl(f, l), fnext, out, qout, qbout, big_deg, s_deg);
+    chunk_push<PM, W>(J, cb, ce - cb, mshfl(f, l), fnext, out, qout, qbout, big_deg, s_deg);
   }
 }
 
@@ -724,7 +724,7 @@ __device__ void qchunk_push(const MsJob& J, uint32_t c0, uint32_t c1, const uint
       f = mld<W>(fcur, ent.x);
     }
     const uint32_t cb = ent.y + (c - ent.w) * CHUNK;
-    chunk_push<PM, W>(J, cb, min(ent.z, cb + CHUNK), f, fnext, out, qout, qbout, big_deg, s_deg);
+    chunk_push<PM, W>(J, cb, min(ent.z - cb, CHUNK), f, fnext, out, qout, qbout, big_deg, s_deg);
   }
 }
 

@@ -219,6 +219,8 @@ int pbg::batch_launch(pbg_batch* b, const pbg_batch_job* jobs, uint32_t njobs, c
       return fail(PBG_ERR_ARG, "one launch takes workspaces of one size class (up to 64, 128 or 256 sources)");
     if (reinterpret_cast<uintptr_t>(J.d_levels) % 16) return fail(PBG_ERR_ARG, "d_levels must be 16-byte aligned");
     if (!seen.insert(J.ws).second) return fail(PBG_ERR_ARG, "a workspace appears twice in one launch");
+    if (J.ws->g->m > PBG_MAX_SEARCH_EDGES)
+      return fail(PBG_ERR_ARG, "searches take at most PBG_MAX_SEARCH_EDGES edges");
     if (J.ws->g->device != b->device) return fail(PBG_ERR_ARG, "job graph on another device");
     if (o.chunk_min_degree < J.ws->big_min_degree)
       return fail(PBG_ERR_ARG, "chunk_min_degree below the one the workspace was sized for");
