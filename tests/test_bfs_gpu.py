@@ -66,6 +66,26 @@ def test_golden_graphs_all_modes(cuda_device, name, case):
     dg.close()
 
 
+@pytest.mark.parametrize("chunk", [1, 32, 1 << 20])
+@pytest.mark.parametrize("name,case", list(golden_cases()))
+def test_golden_graphs_on_the_grid(cuda_device, name, case, chunk):
+    """The golden graphs with isolated vertices up to 6,000, past the one-block search's limit: the same outputs of the
+    reference's own code through the grid's kernels, lists in pieces (1), as the default has it (32), and all walked by
+    one thread each (no list as long as 2^20: the lean kernel)."""
+    n0, n = len(case["offsets"]) - 1, 6000
+    off = np.concatenate([case["offsets"], np.full(n - n0, case["offsets"][-1], np.uint32)])
+    dg = pb.DeviceGraph.upload(off, case["edges"], symmetric=True)
+    for i, s in enumerate(case["srcs"]):
+        s = int(s)
+        for mode in MODES:
+            for d in DIRS:
+                par, _ = check_run(dg, off, case["edges"], s, mode, d, chunk_min_degree=chunk)
+                assert np.all(par[n0:] == -1)
+                if mode == pb.PARENT_MAX:
+                    assert np.array_equal(par[:n0], case["det_max_parent"][i])
+    dg.close()
+
+
 @pytest.mark.parametrize("chunk", [1, 8, 32, 300, 4096])
 @pytest.mark.parametrize("block", [256, 1024])
 def test_degree_bins_and_block_sizes(cuda_device, chunk, block):
@@ -139,6 +159,35 @@ def test_directed_graph_topdown_only(cuda_device):
                                   O.bfs_det_parent(off, edg, 0, "min" if mode == pb.PARENT_MIN else "max"))
     with pytest.raises(pb.PbgError):
         dg.bfs(0, direction=pb.DIR_BOTTOMUP)
+    dg.close()
+
+
+@pytest.mark.parametrize("chunk", [1, 32, 1 << 20])
+def test_directed_graph_on_the_grid(cuda_device, chunk):
+    """A directed graph past the one-block search's limit, with duplicates, self loops and hubs: levels and every rule's
+    parents by the chunked and by the lean kernel."""
+    rng = np.random.default_rng(chunk)
+    n, m = 9001, 50000
+    us = (rng.random(m) ** 2 * n).astype(np.uint32)
+    vs = rng.integers(0, n, m).astype(np.uint32)
+    us[:2000] = 5
+    order = np.lexsort((vs, us))
+    us, vs = us[order], vs[order].copy()
+    off = np.zeros(n + 1, np.int64)
+    np.add.at(off, us.astype(np.int64) + 1, 1)
+    off = np.cumsum(off).astype(np.uint32)
+    dg = pb.DeviceGraph.upload(off, vs, symmetric=False)
+    for src in (0, 5, n - 1):
+        want = levels_of(off, vs, src)
+        for mode in MODES:
+            for d in (pb.DIR_AUTO, pb.DIR_TOPDOWN):
+                par, lv, st = dg.bfs(src, parent_mode=mode, direction=d, levels=True, chunk_min_degree=chunk)
+                assert np.array_equal(lv, want) and st["bottomup_levels"] == 0
+                if mode == pb.PARENT_ANY:
+                    check_parents_by_edges(off, vs, src, par, lv)
+                else:
+                    rule = "min" if mode == pb.PARENT_MIN else "max"
+                    assert np.array_equal(par.view(np.uint32), O.bfs_det_parent(off, vs, src, rule))
     dg.close()
 
 
@@ -297,6 +346,20 @@ def test_dropin_behind_reference_driver_and_checker(cuda_device, tmp_path):
     assert O.check_bfs(off, edg, 0, par) == -1
 
 
+def check_parents_by_edges(off, edg, src, par, levels):
+    """Every reached vertex but the source has a parent one level up with an edge to it, the source itself, and the
+    others none (the checker reads out-edges as in-edges: for directed graphs it cannot say)."""
+    n = len(off) - 1
+    par = par.view(np.uint32)
+    assert par[src] == src
+    assert np.array_equal(par == pb.NONE, levels == pb.NONE)
+    v = np.nonzero((levels != pb.NONE) & (np.arange(n) != src))[0]
+    p = par[v].astype(np.int64)
+    assert np.array_equal(levels[p].astype(np.int64) + 1, levels[v].astype(np.int64))
+    keys = np.repeat(np.arange(n, dtype=np.int64), np.diff(off.astype(np.int64))) * n + edg
+    assert np.isin(p * n + v, keys).all()
+
+
 def _limit_graph(kind, n):
     """Symmetric graphs (and directed ones) of exactly n vertices, the last few isolated."""
     rng = np.random.default_rng(n)
@@ -336,8 +399,9 @@ def test_one_block_search_and_its_limit(cuda_device, kind, n):
                 assert np.array_equal(lv, want), (src, direction, mode)
                 if rule:
                     assert np.array_equal(par.view(np.uint32), O.bfs_det_parent(off, edg, src, rule)), (src, direction, mode)
-                elif sym:
-                    assert O.check_bfs(off, edg, src, par.view(np.uint32)) == -1, (src, direction)
+                else:
+                    check_parents_by_edges(off, edg, src, par, lv)
+                    assert not sym or O.check_bfs(off, edg, src, par.view(np.uint32)) == -1, (src, direction)
                 reached = want != pb.NONE
                 assert st["levels"] == int(want[reached].max()) + 1 and st["visited"] == int(reached.sum())
                 assert st["edges_reached"] == int(deg[reached].sum()) and st["error"] == 0
@@ -351,8 +415,8 @@ def test_one_block_search_and_its_limit(cuda_device, kind, n):
 
 
 def test_one_block_search_edge_limit(cuda_device):
-    """Complete graphs on both sides of the edge limit (searched as directed: the symmetric ones are the grid's), and
-    even lists on both sides of the average that the one block takes."""
+    """Complete graphs on both sides of the edge limit, as directed and as symmetric ones, and random-local graphs of
+    short lists, which the one block takes at any average."""
     for n in (510, 514):  # 259,590 and 263,682 edges around 2^18
         us, vs = np.triu_indices(n, 1)
         off, edg = O.csr_symmetric(n, us.astype(np.uint32), vs.astype(np.uint32))
@@ -395,6 +459,35 @@ def test_host_results_by_either_copy(cuda_device, n):
     pb.check(pb.lib().pbg_bfs(dg.handle, 3, ctypes.byref(opts), pinned.data_ptr(), plain.ctypes.data, None))
     assert np.array_equal(pinned.numpy(), par0) and np.array_equal(plain, lev0)
     dg.close()
+
+
+def test_host_results_of_two_threads(cuda_device):
+    """Two handles, two threads, results large enough for the pinned ring in each call: whoever finds it taken copies
+    plainly, and both get their own results."""
+    import threading
+
+    graphs = [pb.randlocal_graph(n, 2, n // 30, 5) for n in (2_500_003, 3_100_001)]
+    want = [g.bfs(7, parent_mode=pb.PARENT_MIN, levels=True)[:2] for g in graphs]
+    start, wrong = threading.Barrier(2), []
+
+    def work(i):
+        for _ in range(12):
+            start.wait(timeout=60)
+            par, lv, _ = graphs[i].bfs(7, parent_mode=pb.PARENT_MIN, levels=True)
+            if not (np.array_equal(par, want[i][0]) and np.array_equal(lv, want[i][1])):
+                wrong.append(i)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
+    for g, (par, lv) in zip(graphs, want):
+        off, edg = g.download()
+        assert np.array_equal(lv, O.bfs_levels(off, edg, 7))
+        assert np.array_equal(par.view(np.uint32), O.bfs_det_parent(off, edg, 7, "min"))
+        g.close()
 
 
 @pytest.mark.parametrize("side", [False, True])
