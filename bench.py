@@ -1053,8 +1053,8 @@ def run_io(args):
             "cpu_baseline": cpu,
             "e2e": {"value": round(mbs, 1), "unit": "MB/s", "h2d_bytes_per_step": size, "d2h_bytes_per_step": 8,
                     "note": "pbg_graph_load_adj(): file -> pinned pieces -> HBM -> CSR; the same number"},
-            # per load: k_count_tokens, k_parse_tokens, k_validate, k_iso_bitmap (and CUB's scan)
-            "gpu_launches": 4 * args.steps,
+            # per load: k_count_tokens, k_parse_tokens, k_validate (and CUB's scan)
+            "gpu_launches": 3 * args.steps,
         }), flush=True)
     g.close()
 
@@ -1141,8 +1141,9 @@ def run_check(args):
                     "d2h_bytes_per_step": 16,
                     "note": "parents copied from pinned host memory, then pbg_bfs_check (level test)"},
             "cpu_baseline": cpu,
-            # per check: jump_init, one jump_step per doubling round (4 here), jump_finish, check_rows
-            "gpu_launches": 7 * args.steps,
+            # per check: jump_init, 6 jump_step (enqueued ahead, one look; those past the settled round return at
+            # once), jump_finish, check_tails, check_rows
+            "gpu_launches": 10 * args.steps,
             "clocks": clk.summary(),
         }), flush=True)
     dg.close()
@@ -1207,9 +1208,9 @@ def run_build(args):
             "cpu_baseline": cpu,
             "e2e": {"value": round(v, 1), "unit": "M draws/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0,
                     "note": "pbg_graph_generate(): the graph is built and kept in HBM; the same number"},
-            # per graph: k_gen_rmat, k_keys_to_csr, k_validate, k_iso_bitmap (beside CUB's radix sort
-            # and select, about 25 more launches)
-            "gpu_launches": 4 * args.steps,
+            # per graph: k_gen_rmat, k_first_lower, k_lists_below, k_lists_above, k_validate (beside CUB's
+            # radix sorts and select)
+            "gpu_launches": 5 * args.steps,
             "clocks": clk.summary(),
         }), flush=True)
 

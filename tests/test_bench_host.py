@@ -44,3 +44,20 @@ def test_clock_summary_from_nvidia_smi_lines():
 def test_clock_summary_without_samples():
     s = bench.ClockSampler(0).summary()
     assert s["sm_mhz"] is None and s["sm_max_mhz"] is None and s["reasons"] == [] and s["samples"] == 0
+
+
+def test_counted_kernels_exist():
+    """The lines that report own launches as a fixed number a step name the kernels they count: all of them are kernels
+    of the library, and as many as the factor says (a number before a name repeats it)."""
+    import glob
+    import re
+
+    src = "".join(open(f).read() for f in glob.glob(os.path.join(ROOT, "pbbsbench_b200", "csrc", "*.cu")))
+    kernels = set(re.findall(r"__global__\s+void\s+(?:__launch_bounds__\([^)]*\)\s+)?(\w+)\s*\(", src))
+    text = open(os.path.join(ROOT, "bench.py")).read()
+    counted = re.findall(r"((?:^ *#[^\n]*\n)+) *\"gpu_launches\": (\d+) \* args\.steps", text, flags=re.M)
+    assert len(counted) >= 3
+    for comment, factor in counted:
+        named = re.findall(r"(?:(\d+) )?\b((?:k|jump|check|strip)_\w+)", comment)
+        assert named and {k for _, k in named} <= kernels, comment
+        assert sum(int(c or 1) for c, _ in named) == int(factor), comment
