@@ -263,8 +263,8 @@ class DeviceGraph:
         return st.as_dict()
 
     def mis_trace(self) -> list:
-        """Per-round trace of the last MIS: vertices walked and device time
-        of each round."""
+        """Trace of the last MIS, one entry per pass (there is one): vertices
+        walked and device time."""
         return _read_trace(lib().pbg_mis_trace, self._h)
 
     def trace_multi(self) -> list:

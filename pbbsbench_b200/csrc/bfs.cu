@@ -135,8 +135,12 @@ __device__ __forceinline__ void load_ranges(const BfsArgs& a, const uint32_t (&v
 // which costs a select each and keeps some 20 registers free for the loops.
 // The 1024-thread kernels are held to 64 registers: with this and 32-bit
 // per-thread sums they spill 136-140 bytes (bfs_lean 72) instead of 244-280
-// (196-240); torus 160^3 1.677 -> 1.622 ms, rMat 2^24 0.562 -> 0.547 ms,
-// rMat 2^12 53.2 -> 51.2 us.
+// (196-240).  us a search, before and now, same box, runs within 0.2%: rMat
+// 2^24 561 / 551, 2^20 64.4 / 61.5; bfs_lean, ANY: torus 160^3 1659 / 1600,
+// 100^3 881 / 877, 60^3 507 / 505, 40^3 356 / 327, 20^3 163 / 166; random-local
+// 100 k 302 / 303, 1 M 622 / 636, 8 M 2615 / 2660: wide levels of short lists
+// pay the selects without having had spills in the way.  Carrying the queue
+// pointers again there costs the lattices more (torus 160^3 1659).
 struct Level {
   uint32_t bits;  // 0: output queues are q0/qr0/qb0 (else q1/qr1/qb1); 1: bm1 is the visited bitmap
   uint32_t slot;  // counters of the frontier produced (3: conv)
@@ -915,8 +919,13 @@ constexpr uint16_t NO_LEVEL = 0xFFFF;
 // 2^12, 16n 53.0 / 29.7; 2^12, 30n 49.2 / 31.8; torus 17^3 131 / 73; randLocal
 // 5101, 3 edges within 60 420 / 130, 8 within 700 69.6 / 58.3, 20 within 700
 // 81.6 / 70.2, 25 within 100 257 / 162; directed 5101, 61 k edges 70.9 / 70.3,
-// 121 k 125 / 104.  Past the line: randLocal 8001, 8 edges within 1000 76 / 94;
-// rMat 2^13, 14n 53 / 52; directed 8001, 96 k edges 97 / 103.
+// 121 k 125 / 104.  Past the line, grid / one block built with a limit of 8,192
+// (whose wider bottom-up step spills 50-96 bytes): randLocal 6001, 8 edges
+// within 700 79 / 87; 7001, 8 within 900 68 / 85, 20 within 700 98 / 98; 8001, 8
+// within 1000 73 / 85; rMat 2^13, 14n 39 / 40; directed 8001, 96 k edges 97 /
+// 103; but graphs of many small levels gain there too: torus 18^3 152 / 83,
+// 20^3 166 / 98, randLocal 6001, 3 within 60 438 / 153.  Vertices and edges do
+// not tell the two kinds apart, so the line is where no kind loses.
 bool small_graph(const pbg_graph* g) { return g->n <= SMALL_N && g->m <= SMALL_M; }
 
 size_t small_bytes(uint32_t n, uint32_t nwords) {

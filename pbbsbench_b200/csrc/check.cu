@@ -210,9 +210,11 @@ __global__ void check_rows(const uint32_t* __restrict__ off, const uint32_t* __r
 // pieces need no byte-wise atomic minimum.  n >= 256 is assumed: 255 in a
 // strip is "unreached" and nothing else.
 //
-// Bound by the L2's sector rate of the strip gathers (S bytes an edge).
-// 64 rows on rMat 2^20 (m = 31.4 M): 21.2 ms a row at a time, now 0.55 ms (the
-// transpose 0.066, tails 0.25, lists 0.23: 5.3 TB/s of strip gathers).
+// Bound by instruction issue: the byte minima and compares (four bytes an
+// instruction, several instructions each) keep the ALU pipe 67-70% busy, with
+// the gathers' L2 traffic at 12-25% of its rate.  64 rows on rMat 2^20 (m = 31.4
+// M): 21.2 ms a row at a time, now 0.58 ms (the transpose 0.067, tails 0.26,
+// lists 0.24).
 
 // rows [0, rows) of n bytes -> strips of `stride` bytes; rows past the last
 // read as 255.  One block: 128 vertices, through shared memory.

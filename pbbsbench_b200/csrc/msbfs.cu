@@ -180,9 +180,10 @@ __device__ __forceinline__ Mask<W> mshfl(const Mask<W>& m, int src) {
 // OR over the warp, by warp reductions of the 32-bit halves: two instructions
 // a word instead of 20 (five 64-bit shuffles).  Level sums of a warp (at most
 // m < 2^32 edges) are reduced in 32 bits the same way.  These ran several
-// times a 32-vertex tile: 64 sources on randLocal 2^23 26.86 -> 25.87 ms,
-// eight rMat graphs 2^16-2^23 fused 5.00 -> 4.80 ms, 256 sources on rMat 2^20
-// 1.517 -> 1.475 ms.
+// times a 32-vertex tile.  Same graphs and sources, in turn: 64 sources on
+// randLocal 2^23 26.98 -> 25.96 ms, eight rMat graphs 2^16-2^23 fused 5.36 ->
+// 5.16 ms (runs of one side differ by 1.2%), 256 sources on rMat 2^20 1.741 ->
+// 1.717 ms.
 template <int W>
 __device__ __forceinline__ Mask<W> warp_or(Mask<W> m) {
 #pragma unroll
