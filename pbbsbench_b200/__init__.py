@@ -94,9 +94,10 @@ class DeviceGraph:
             check(lib().pbg_graph_upload(_ptr(offsets), _ptr(edges), len(offsets) - 1, int(offsets[-1]), flags,
                                          ctypes.byref(h)))
         else:  # torch tensors on the device
-            if offsets.is_cuda:  # what fills them may still be queued on a stream that the copies do not wait for
+            if getattr(offsets, "is_cuda", False):
                 import torch
 
+                # what fills them may still be queued on a stream that the copies do not wait for
                 torch.cuda.current_stream(offsets.device).synchronize()
             check(lib().pbg_graph_upload_device(_ptr(offsets), _ptr(edges), offsets.numel() - 1, edges.numel(),
                                                 flags, ctypes.byref(h)))
